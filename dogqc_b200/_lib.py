@@ -132,6 +132,11 @@ NOALLOC_MAX_BUILD_ROWS = 262144
 NOALLOC_MAX_GROUPS = 4096
 
 
+class dq_result_col(C.Structure):
+    _fields_ = [("ctype", C.c_int32), ("reserved", C.c_int32), ("data", C.c_void_p), ("bytes", C.c_uint64),
+                ("chars", C.c_void_p), ("nchars", C.c_uint64)]
+
+
 class dq_join_agg_args(C.Structure):
     _fields_ = [("build_key", C.c_void_p), ("build_filter", C.c_void_p), ("filter_value", C.c_int32),
                 ("build_group", C.c_void_p), ("build_rows", C.c_int64), ("probe_key", C.c_void_p),
@@ -144,7 +149,7 @@ def check_layout():
     """Sizes the C compiler gives these structs on x86-64 (LP64)."""
     expect = {dq_config: 40, dq_column: 40, dq_slot: 8, dq_op: 40, dq_resource: 80, dq_join_agg_args: 104,
               dq_tuning: 32, dq_server_config: 32, dq_request_info: 40, dq_server_stats: 88,
-              dq_text_field: 16, dq_import_timing: 72}
+              dq_text_field: 16, dq_import_timing: 72, dq_result_col: 40}
     for t, n in expect.items():
         if C.sizeof(t) != n:
             raise AssertionError("%s is %d bytes, header implies %d" % (t.__name__, C.sizeof(t), n))
@@ -184,6 +189,7 @@ EXPORTS = {
     "dq_result_ncols": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32)]),
     "dq_result_column": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_int32), C.POINTER(C.c_void_p)]),
     "dq_result_string_heap": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_void_p), C.POINTER(C.c_uint64)]),
+    "dq_result_view": (C.c_int, [C.c_void_p, C.POINTER(C.c_int64), C.POINTER(C.c_int32), C.POINTER(dq_result_col)]),
     "dq_result_free": (None, [C.c_void_p]),
     "dq_join_agg_noalloc": (C.c_int, [C.POINTER(dq_join_agg_args), C.c_void_p]),
     "dq_plan_prepare_tuned": (C.c_int, [C.c_void_p, C.POINTER(dq_plan_desc), C.POINTER(dq_tuning),

@@ -204,15 +204,57 @@ struct DevPipe {
 // A batch runs many instances of one plan shape: these descriptors let one
 // launch reset, scan or pack the per-instance buffers of all instances.
 
-struct BatchReset {       // one buffer to reset before a batch run
+constexpr uint64_t kResetChunk = 8192;  // 64-bit words one CTA resets at a time
+
+struct BatchReset {       // one buffer to reset before a run (8-byte aligned)
   void* ptr;
-  uint64_t n;             // 64-bit words (kind 0), 32-bit words (kind 1), slots (kind 2)
-  uint64_t value;         // kinds 0 and 1
-  uint64_t reds;          // kind 2: 4 bits of dq_red_kind per aggregate
-  int32_t kind;           // 0: fill u64, 1: fill u32, 2: aggregation table
-  int32_t words;          // kind 2: words per slot
-  int32_t val_word;       // kind 2: first accumulator word
-  int32_t naggs;          // kind 2
+  uint64_t n;             // 64-bit words
+  uint64_t value;         // kind 0
+  uint64_t reds;          // kind 1: 4 bits of dq_red_kind per aggregate
+  uint64_t chunk0;        // its first chunk of kResetChunk words among all buffers'
+  int32_t kind;           // 0: fill u64, 1: aggregation table
+  int32_t words;          // kind 1: words per slot
+  int32_t val_word;       // kind 1: first accumulator word
+  int32_t naggs;          // kind 1
+};
+
+// The buffers a plan's run starts by resetting, as a kernel parameter.
+constexpr int kMaxResets = 48;
+struct ResetList {
+  int32_t n;
+  int32_t pad;
+  uint64_t chunks;
+  BatchReset op[kMaxResets];
+};
+
+// A run's status word, row count and result columns in pinned host memory:
+// the header, then a region per column.  A column that does not fit its region
+// (more rows, longer strings) is copied by the host after the run.
+constexpr uint64_t kPackBytes = 32768;  // bytes a column's region holds at most
+constexpr uint32_t kPackRows = 2048;    // rows of a string column at most
+constexpr int kPackHeader = 256;        // int32 status, uint64 rows at 8, uint64 heap
+                                        // bytes of string column j at 16 + 8 j (~0: too large)
+
+struct ResultPackCol {
+  const uint8_t* src;
+  uint64_t off;           // its region's offset (strings: the offsets, then kPackBytes of heap)
+  uint64_t bytes;         // a fixed-width region's size
+  int32_t width;          // 0: string references
+  int32_t heap_off;       // strings: the heap's offset in the region
+};
+
+constexpr int kMaxPackStats = 8;
+struct ResultPack {
+  const int32_t* status;
+  const uint64_t* cursor;
+  uint64_t cap;
+  const DevStr* strsrc;
+  uint8_t* out;
+  int32_t ncols;
+  int32_t nstats;         // pairs of counters copied beside the result (deferred items)
+  const uint32_t* stat_src[kMaxPackStats];
+  uint32_t* stat_dst[kMaxPackStats];
+  ResultPackCol c[DQ_MAX_PAY];
 };
 
 struct BatchScanSeg {     // one multimap's bucket counts -> offsets

@@ -1207,21 +1207,6 @@ __global__ void __launch_bounds__(kThreads, 3) row_kernel(const __grid_constant_
 
 // ------------------------------------------------------- helper kernels --
 
-// Fills aggregation tables: tags empty, accumulators at their initial values.
-__global__ void agg_init_kernel(uint64_t* slots, uint64_t nslots, int words, int val_word, int naggs,
-                                uint64_t red_packed) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nslots * words;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t w = i % words;
-    uint64_t v = kEmpty;
-    if ((int)w >= val_word && (int)w < val_word + naggs) {
-      int red = (int)((red_packed >> (4 * (w - val_word))) & 15);
-      v = red_init(red);
-    }
-    slots[i] = v;
-  }
-}
-
 // Multimap bucket offsets: exclusive scan of counts in three passes.
 constexpr int kScanItems = 16;
 constexpr int kScanChunk = kThreads * kScanItems;
@@ -1450,24 +1435,34 @@ __global__ void heavy_group_scatter_kernel(DevHeavy H) {
 
 // ------------------------------------------------------- batch helpers --
 
-// Resets every per-instance buffer of a batch in one launch; each CTA walks
-// all descriptors (starting at a rotated one) and strides over its share.
-__global__ void batch_reset_kernel(const BatchReset* ops, int nops) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (int k = 0; k < nops; ++k) {
-    const int o = (int)((blockIdx.x + (unsigned)k) % (unsigned)nops);
-    const BatchReset op = ops[o];
-    const uint64_t start = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Resets many buffers in one launch.  The buffers' chunks (kResetChunk words)
+// are numbered through; a CTA takes chunks grid-stride and finds each one's
+// buffer by its first chunk, so small buffers cost one CTA a chunk and a large
+// one is spread over the grid.  Bound by the writes (16 bytes a thread and
+// store) or, for a plan's few small tables, by one kernel's latency instead of
+// one memset's after the other.
+__device__ __forceinline__ void reset_chunks(const BatchReset* ops, int nops, uint64_t nchunks) {
+  for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+    int lo = 0, hi = nops;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (ops[mid].chunk0 <= c) lo = mid;
+      else hi = mid;
+    }
+    const BatchReset op = ops[lo];
+    const uint64_t w0 = (c - op.chunk0) * kResetChunk;
+    const uint64_t w1 = w0 + kResetChunk < op.n ? w0 + kResetChunk : op.n;
+    uint64_t* const p = reinterpret_cast<uint64_t*>(op.ptr);
     if (op.kind == 0) {
-      uint64_t* p = reinterpret_cast<uint64_t*>(op.ptr);
-      for (uint64_t i = start; i < op.n; i += stride) p[i] = op.value;
-    } else if (op.kind == 1) {
-      uint32_t* p = reinterpret_cast<uint32_t*>(op.ptr);
-      for (uint64_t i = start; i < op.n; i += stride) p[i] = (uint32_t)op.value;
+      if ((reinterpret_cast<uint64_t>(p) & 15) == 0) {
+        const ulonglong2 v = make_ulonglong2(op.value, op.value);
+        for (uint64_t i = w0 + 2 * threadIdx.x; i + 1 < w1; i += 2 * blockDim.x) *reinterpret_cast<ulonglong2*>(p + i) = v;
+        if (threadIdx.x == 0 && ((w1 - w0) & 1)) p[w1 - 1] = op.value;
+      } else {
+        for (uint64_t i = w0 + threadIdx.x; i < w1; i += blockDim.x) p[i] = op.value;
+      }
     } else {
-      uint64_t* p = reinterpret_cast<uint64_t*>(op.ptr);
-      const uint64_t total = op.n * (uint64_t)op.words;
-      for (uint64_t i = start; i < total; i += stride) {
+      for (uint64_t i = w0 + threadIdx.x; i < w1; i += blockDim.x) {
         const int w = (int)(i % (uint64_t)op.words);
         uint64_t v = kEmpty;
         if (w >= op.val_word && w < op.val_word + op.naggs) v = red_init((int)((op.reds >> (4 * (w - op.val_word))) & 15));
@@ -1475,6 +1470,81 @@ __global__ void batch_reset_kernel(const BatchReset* ops, int nops) {
       }
     }
   }
+}
+
+__global__ void batch_reset_kernel(const BatchReset* ops, int nops, uint64_t nchunks) { reset_chunks(ops, nops, nchunks); }
+
+__global__ void reset_kernel(const __grid_constant__ ResetList L) { reset_chunks(L.op, L.n, L.chunks); }
+
+// A run's status, row count and result columns written to pinned host memory,
+// a CTA per column (the last launch of a run: the host reads the result after
+// one wait, with no copy per column).  String columns: offsets from a block
+// scan of the lengths, the bytes gathered in shared memory and written in
+// 16-byte stores.
+__global__ void __launch_bounds__(kThreads) result_pack_kernel(const __grid_constant__ ResultPack A) {
+  extern __shared__ __align__(16) uint8_t heap[];  // kPackBytes, when a column is a string
+  __shared__ uint32_t soff[kPackRows + 1];
+  const int tid = threadIdx.x;
+  const int32_t status = *A.status;
+  uint64_t n = A.cursor ? *A.cursor : 0;
+  if (n > A.cap) n = A.cap;
+  if (blockIdx.x == 0) {
+    if (tid == 0) {
+      *reinterpret_cast<int32_t*>(A.out) = status;
+      *reinterpret_cast<uint64_t*>(A.out + 8) = n;
+    }
+    if (tid < 2 * A.nstats) A.stat_dst[tid >> 1][tid & 1] = A.stat_src[tid >> 1][tid & 1];
+  }
+  if ((status & ~kInfoMask) || (int)blockIdx.x >= A.ncols) return;
+  const ResultPackCol& c = A.c[blockIdx.x];
+  uint8_t* const dst = A.out + c.off;
+  if (c.width > 0) {
+    const uint64_t bytes = n * (uint64_t)c.width;
+    if (bytes > c.bytes) return;
+    for (uint64_t i = (uint64_t)tid * 16; i < bytes; i += kThreads * 16)
+      *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(c.src + i);
+    return;
+  }
+  uint64_t* const heap_bytes = reinterpret_cast<uint64_t*>(A.out + 16) + blockIdx.x;
+  if (n > kPackRows) {
+    if (tid == 0) *heap_bytes = ~0ull;
+    return;
+  }
+  const uint64_t* const refs = reinterpret_cast<const uint64_t*>(c.src);
+  uint64_t* const offs = reinterpret_cast<uint64_t*>(dst);
+  uint32_t carry = 0;
+  for (uint32_t base = 0; base < (uint32_t)n; base += kThreads) {
+    const uint32_t r = base + tid;
+    uint32_t len = 0;
+    if (r < (uint32_t)n) {
+      const uint8_t* p;
+      int m;
+      str_ref_bytes(A.strsrc, refs[r], p, m);
+      len = m < (int)kPackBytes + 1 ? (uint32_t)m : (uint32_t)kPackBytes + 1;  // the sum cannot wrap
+    }
+    uint32_t excl;
+    const uint32_t total = block_exclusive_scan(len, excl);
+    if (r < (uint32_t)n) {
+      soff[r] = carry + excl;
+      offs[r] = carry + excl;
+    }
+    carry += total;
+  }
+  if (tid == 0) {
+    offs[n] = carry;
+    *heap_bytes = carry <= kPackBytes ? carry : ~0ull;
+  }
+  if (carry > kPackBytes) return;
+  __syncthreads();
+  for (uint32_t r = tid >> 5; r < (uint32_t)n; r += kThreads / 32) {
+    const uint8_t* p;
+    int m;
+    str_ref_bytes(A.strsrc, refs[r], p, m);
+    for (int i = tid & 31; i < m; i += 32) heap[soff[r] + i] = p[i];
+  }
+  __syncthreads();
+  for (uint32_t i = tid * 16; i < carry; i += kThreads * 16)
+    *reinterpret_cast<uint4*>(dst + c.heap_off + i) = *reinterpret_cast<const uint4*>(heap + i);
 }
 
 __device__ __forceinline__ int batch_seg_of(const BatchScanSeg* segs, int nseg, uint64_t block) {
@@ -1586,18 +1656,6 @@ int pipeline_occupancy(int smem_bytes) {
   return blocks;
 }
 
-cudaError_t launch_agg_init(uint64_t* slots, uint64_t nslots, int words, int val_word, int naggs,
-                            const int8_t* reds, cudaStream_t stream) {
-  uint64_t packed = 0;
-  for (int j = 0; j < naggs && j < 16; ++j) packed |= (uint64_t)(reds[j] & 15) << (4 * j);
-  uint64_t total = nslots * words;
-  uint64_t want = (total + 255) / 256;
-  int grid = (int)(want < 148ull * 16 ? want : 148ull * 16);
-  if (grid < 1) grid = 1;
-  agg_init_kernel<<<grid, 256, 0, stream>>>(slots, nslots, words, val_word, naggs, packed);
-  return cudaGetLastError();
-}
-
 size_t mm_scan_scratch_words(uint64_t n) { return (n + kScanChunk - 1) / kScanChunk + 1; }
 
 cudaError_t launch_mm_scan(uint32_t* counts, uint32_t* offsets, uint64_t n, uint32_t* partials,
@@ -1613,9 +1671,24 @@ cudaError_t launch_mm_scan(uint32_t* counts, uint32_t* offsets, uint64_t n, uint
 
 size_t batch_scan_blocks(uint64_t n) { return (size_t)((n + kScanChunk - 1) / kScanChunk); }
 
-cudaError_t launch_batch_reset(const BatchReset* ops, int nops, int sms, cudaStream_t stream) {
-  if (nops <= 0) return cudaSuccess;
-  batch_reset_kernel<<<sms * 4, 256, 0, stream>>>(ops, nops);
+cudaError_t launch_batch_reset(const BatchReset* ops, int nops, uint64_t nchunks, int sms, cudaStream_t stream) {
+  if (nops <= 0 || nchunks == 0) return cudaSuccess;
+  const uint64_t most = (uint64_t)sms * 8;
+  batch_reset_kernel<<<(unsigned)(nchunks < most ? nchunks : most), 256, 0, stream>>>(ops, nops, nchunks);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_resets(const ResetList& L, int sms, cudaStream_t stream) {
+  if (L.n <= 0 || L.chunks == 0) return cudaSuccess;
+  const uint64_t most = (uint64_t)sms * 8;
+  reset_kernel<<<(unsigned)(L.chunks < most ? L.chunks : most), 256, 0, stream>>>(L);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_result_pack(const ResultPack& A, cudaStream_t stream) {
+  bool strings = false;
+  for (int j = 0; j < A.ncols; ++j) strings |= A.c[j].width == 0;
+  result_pack_kernel<<<A.ncols > 0 ? A.ncols : 1, kThreads, strings ? kPackBytes : 0, stream>>>(A);
   return cudaGetLastError();
 }
 

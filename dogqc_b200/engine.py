@@ -55,37 +55,49 @@ class Result(object):
         return "\n".join(out) + "\n"
 
 
+_NP_DTYPES = {t: np.dtype(d) for t, d in NP_DTYPE.items()}
+_OFFSETS = np.dtype(np.uint64)
+_BYTES = np.dtype(np.uint8)
+
+
+def _copied(ptr, nbytes, dtype):
+    """A writable numpy array of its own of the nbytes at ptr."""
+    if nbytes <= 4096:  # a copy through bytes costs less than looking up an array's address
+        return np.frombuffer(bytearray(C.string_at(ptr, nbytes)) if nbytes else bytearray(), dtype)
+    out = np.empty(nbytes // dtype.itemsize, dtype)
+    C.memmove(out.__array_interface__["data"][0], ptr, nbytes)
+    return out
+
+
+def _take_results(handles, names):
+    """Copies dq_results into Results and frees them (all of them, also when one
+    cannot be read); names: the column names of each."""
+    lib = L.lib()
+    n, nc, view = C.c_int64(), C.c_int32(), (L.dq_result_col * L.MAX_PAY)()
+    pn, pc = C.byref(n), C.byref(nc)
+    out = []
+    try:
+        for at, res in enumerate(handles):
+            L.check(lib.dq_result_view(res, pn, pc, view))
+            cols, types = [], []
+            for j in range(nc.value):
+                c = view[j]
+                t = c.ctype
+                types.append(t)
+                if t == L.STR:  # offsets into a heap, kept as a StringColumn (bytes per row on demand)
+                    cols.append(StringColumn(_copied(c.chars, c.nchars, _BYTES), _copied(c.data, c.bytes, _OFFSETS)))
+                else:
+                    cols.append(_copied(c.data, c.bytes, _NP_DTYPES[t]))
+            out.append(Result(names[at], types, cols, n.value))
+    finally:
+        for res in handles:
+            lib.dq_result_free(res)
+    return out
+
+
 def _take_result(res, names):
     """Copies a dq_result into a Result and frees it."""
-    lib = L.lib()
-    try:
-        n = C.c_int64()
-        nc = C.c_int32()
-        L.check(lib.dq_result_rows(res, C.byref(n)))
-        L.check(lib.dq_result_ncols(res, C.byref(nc)))
-        cols, types = [], []
-        for j in range(nc.value):
-            t = C.c_int32()
-            ptr = C.c_void_p()
-            L.check(lib.dq_result_column(res, j, C.byref(t), C.byref(ptr)))
-            if t.value == L.STR:  # offsets into a heap, kept as a StringColumn (bytes per row on demand)
-                offs = np.frombuffer((C.c_uint8 * ((n.value + 1) * 8)).from_address(ptr.value), np.uint64).copy()
-                hp, nch = C.c_void_p(), C.c_uint64()
-                L.check(lib.dq_result_string_heap(res, j, C.byref(hp), C.byref(nch)))
-                heap = C.string_at(hp.value, nch.value) if nch.value else b""
-                cols.append(StringColumn(np.frombuffer(heap, dtype=np.uint8), offs))
-                types.append(t.value)
-                continue
-            dt = np.dtype(NP_DTYPE[t.value])
-            if n.value:
-                buf = (C.c_uint8 * (n.value * dt.itemsize)).from_address(ptr.value)
-                cols.append(np.frombuffer(buf, dtype=dt).copy())
-            else:
-                cols.append(np.zeros(0, dtype=dt))
-            types.append(t.value)
-    finally:
-        lib.dq_result_free(res)
-    return Result(names, types, cols, n.value)
+    return _take_results([res], [names])[0]
 
 
 def make_tuning(tuning):
@@ -190,7 +202,7 @@ class Batch(object):
         n = len(self.lowerings)
         out = (C.c_void_p * n)()
         L.check(L.lib().dq_batch_execute(self.handle, stream, out), self.engine.ctx)
-        return [_take_result(C.c_void_p(out[i]), self.lowerings[i].result_names) for i in range(n)]
+        return _take_results(list(out), [lw.result_names for lw in self.lowerings])
 
     def profile(self, point):
         """Lane-activity histogram of profile point ``point`` in the last

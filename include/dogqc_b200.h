@@ -485,6 +485,17 @@ int dq_result_column(dq_result* r, int32_t col, int32_t* ctype, const void** dat
 /* A DQ_STR result column: dq_result_column gives nrows+1 uint64 offsets into
  * this heap of `*nchars` bytes.                                              */
 int dq_result_string_heap(dq_result* r, int32_t col, const void** chars, uint64_t* nchars);
+/* A whole result in one call: its rows and columns (as dq_result_column and
+ * dq_result_string_heap give them) into cols, which holds DQ_MAX_PAY entries.  */
+typedef struct {
+    int32_t ctype;
+    int32_t reserved;
+    const void* data;
+    uint64_t bytes;
+    const void* chars;               /* DQ_STR: the heap                         */
+    uint64_t nchars;
+} dq_result_col;
+int dq_result_view(dq_result* r, int64_t* nrows, int32_t* ncols, dq_result_col* cols);
 void dq_result_free(dq_result* r);
 
 /* ------------------------------------------------- allocation-free join -- */
