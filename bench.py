@@ -152,7 +152,8 @@ def pipeline_bytes(db, lowering, i):
 
 
 def join_pairs(db):
-    """Matching (probe, build) key pairs of the divergent-expansion workload."""
+    """Matching (probe, build) key pairs of the divergent-expansion workload's
+    join, before its filters (which read the build side only and run there)."""
     import numpy as np
     b = np.bincount(db["r_build"].columns["r_key"])
     p = np.bincount(db["s_probe"].columns["s_key"])
