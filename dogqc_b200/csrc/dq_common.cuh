@@ -820,6 +820,31 @@ __device__ __forceinline__ int local_group_slot(uint64_t* tags, int ns, uint64_t
   return -1;
 }
 
+// The same table when few groups are expected: ns (a power of two) is several
+// times their number, so a group is mostly found at its home slot, from a
+// 32-bit hash of the tag's halves.  The claimer numbers the group (ids[slot],
+// kEmpty32 until then): groups with a small number have accumulators of their
+// own per thread.
+__device__ __forceinline__ int local_group_slot_id(uint64_t* tags, uint32_t* ids, uint32_t* nids, int ns, int shift,
+                                                   uint64_t tag) {
+  if (tag == kEmpty) {
+    s_cas64(saddr(&tags[ns]), kEmpty, 0ull);
+    return ns;
+  }
+  uint32_t idx = ((uint32_t)tag * 0x9e3779b1u ^ (uint32_t)(tag >> 32) * 0x85ebca77u) >> shift;
+  for (int n = 0; n < ns; ++n) {
+    const uint64_t t = ((volatile uint64_t*)tags)[idx];
+    if (t == tag) return (int)idx;
+    if (t == kEmpty) {
+      const uint64_t old = s_cas64(saddr(&tags[idx]), kEmpty, tag);
+      if (old == kEmpty) ((volatile uint32_t*)ids)[idx] = atomicAdd(nids, 1u);
+      if (old == kEmpty || old == tag) return (int)idx;
+    }
+    idx = (idx + 1) & (uint32_t)(ns - 1);
+  }
+  return -1;
+}
+
 // CTA-local group table for hashed keys that include strings: tags, then the
 // keys (string references) of each slot.  A claim publishes the keys before
 // the tag; a match compares the keys (strings by their bytes).  -1 when the

@@ -107,6 +107,7 @@ struct DevRes {
   uint8_t* pay[DQ_MAX_PAY];   // MULTI payload columns / OUTPUT columns
   uint64_t* cursor;       // OUTPUT row cursor
   int32_t smem_slots;     // AGG: CTA-local table slots (0: global only)
+  int32_t group_hint;     // AGG: groups the plan expects
   int32_t smem_off;       // AGG: offset of the CTA-local table
   int32_t bitmap;         // UNIQUE over a small key domain [bmin, bmin + brange):
                           // 1: no payload, slots hold one bit per key;

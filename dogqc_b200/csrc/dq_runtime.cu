@@ -595,6 +595,7 @@ void setup_resource(dq_plan* plan, ResRec& r, int64_t build_rows_bound) {
         uint64_t bytes = (ns + 1) * (1 + d.naggs) * 8 + (str_keys ? ns * d.nkeys * 8 : 0);
         if (d.nkeys == 0) ns = 1, bytes = 2 * (1 + d.naggs) * 8;
         R.smem_slots = bytes <= 24 * 1024 ? (int)ns : 0;
+        R.group_hint = (int32_t)std::min<int64_t>(std::max<int64_t>(d.group_hint, 0), 1 << 30);
       }
       break;
     }
