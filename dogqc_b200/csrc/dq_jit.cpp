@@ -477,6 +477,45 @@ struct Gen {
       }
   }
 
+  // The literals of a LIKE pattern '%L1%...%Ln%' (no '_', no empty literal) as
+  // (offset in the pattern buffer, length); none for other patterns.
+  std::vector<std::pair<int, int>> like_literals(int pattern) const {
+    std::vector<std::pair<int, int>> lits;
+    if (!patterns) return lits;
+    const int o = P.pat_off[pattern], lp = P.pat_off[pattern + 1] - o;
+    const std::string pat = patterns->substr((size_t)o, (size_t)lp);
+    if (lp < 3 || pat.front() != '%' || pat.back() != '%' || pat.find('_') != std::string::npos) return lits;
+    for (int i = 1, start = 1; i < lp; ++i)
+      if (pat[(size_t)i] == '%') {
+        if (i == start) return {};
+        lits.emplace_back(o + start, i - start);
+        start = i + 1;
+      }
+    return lits;
+  }
+
+  // The literal of LIKE op k that the whole warp looks for first (an index into
+  // its literals), or -1: the op reads a column in place before any operator
+  // has dropped rows, so the warp's lanes hold consecutive strings (one row a
+  // lane and step: generate() then takes U = 1), and the literal has at least
+  // three bytes.
+  int scan_literal(int k) const {
+    const dq_op& op = P.ops[k];
+    if (op.kind != DQ_OP_LIKE || slot(op.a).kind != DQ_SLOT_STR || P.source_kind != DQ_SRC_TABLE) return -1;
+    for (int j = 0; j < k; ++j)
+      switch (P.ops[j].kind) {
+        case DQ_OP_FILTER:
+        case DQ_OP_PROBE:
+        case DQ_OP_EXISTS:
+        case DQ_OP_EXPAND:
+          return -1;
+      }
+    const auto lits = like_literals(op.res);
+    for (size_t i = 0; i < lits.size(); ++i)
+      if (lits[i].second >= 3) return (int)i;
+    return -1;
+  }
+
   void skip_if_idle(const std::string& act, const std::string& exit) {
     L("if (!__any_sync(kFull, " + act + ")) " + exit);
   }
@@ -534,20 +573,32 @@ struct Gen {
           break;
         case DQ_OP_LIKE: {
           // a pattern '%L1%...%Ln%' (no '_', no empty literal) finds its
-          // literals one after another, eight bytes a step; others run the
-          // reference matcher's algorithm (like_match)
-          std::vector<std::pair<int, int>> lits;  // (offset in the pattern buffer, length)
-          bool simple = false;
-          if (patterns) {
-            const int o = P.pat_off[op.res], lp = P.pat_off[op.res + 1] - o;
-            const std::string pat = patterns->substr((size_t)o, (size_t)lp);
-            simple = lp >= 3 && pat.front() == '%' && pat.back() == '%' && pat.find('_') == std::string::npos;
-            for (int i = 1, start = 1; simple && i < lp; ++i)
-              if (pat[(size_t)i] == '%') {
-                if (i == start) simple = false;
-                else lits.emplace_back(o + start, i - start);
-                start = i + 1;
-              }
+          // literals one after another, eight bytes a step, in the strings
+          // that can hold one of them; others run the reference matcher's
+          // algorithm (like_match)
+          const std::vector<std::pair<int, int>> lits = like_literals(op.res);
+          const bool simple = !lits.empty();
+          const int scan = U == 1 && row == "row" ? scan_literal(k) : -1;
+          if (scan >= 0) {
+            const std::string id = num(uid++);
+            L("const uint8_t* lk" + id + "_ = nullptr; int ln" + id + "_ = 0;");
+            L("if (" + act + ") str_at(P.strs[" + num(slot(op.a).src) + "], row, lk" + id + "_, ln" + id + "_);");
+            L("bool lc" + id + "_ = false;");
+            L("if (__any_sync(kFull, " + act + "))");
+            L("  lc" + id + "_ = like_candidates(" + act + ", lk" + id + "_, ln" + id + "_, P.patterns + " + num(lits[(size_t)scan].first) +
+              ", " + num(lits[(size_t)scan].second) + ");");
+            L(V(op.dst) + " = 0;");
+            L("if (lc" + id + "_) {");
+            ++ind;
+            L("int lp_ = 0;");
+            std::string cond;
+            for (auto& l : lits)
+              cond += (cond.empty() ? "" : " && ") + ("like_find(lk" + id + "_, ln" + id + "_, lp_, P.patterns + ") + num(l.first) +
+                      ", " + num(l.second) + ")";
+            L(V(op.dst) + " = (uint64_t)(" + cond + ");");
+            --ind;
+            L("}");
+            break;
           }
           L(V(op.dst) + " = 0;");
           L("if (" + act + ") {");
@@ -2302,6 +2353,10 @@ Program generate(const DevPipe& P, int expand_op, int refill_op, const Tuning& t
   if (rows > 0 && !has_expand && P.source_kind != DQ_SRC_AGG) g.U = rows >= 4 ? 4 : rows >= 2 ? 2 : 1;
   if (t.refill < 0) refill_op = -1;
   if (t.refill_threshold >= 1 && t.refill_threshold <= 32) g.refill_threshold = t.refill_threshold;
+  // strings searched by the whole warp: consecutive rows on consecutive lanes
+  bool scans = false;
+  for (int k = 0; k < P.nops; ++k) scans |= g.scan_literal(k) >= 0;
+  if (scans) g.U = 1;
   g.choose_agg();
   g.choose_refill(refill_op);
   g.choose_hot();
