@@ -230,17 +230,23 @@ __device__ __forceinline__ void prefetch_bytes(const uint8_t* p, int n) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(a + 128ull * (unsigned long long)i));
 }
 
+// The low min(m, 4) bytes of a 32-bit word (m <= 0: none).
+__device__ __forceinline__ uint32_t low_bytes(uint32_t w, int m) {
+  uint32_t mask;
+  asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(mask) : "r"(8 * (m > 0 ? m : 0)));
+  return w & mask;
+}
+
 // Bytes p[0, m) (1 <= m <= 8) as a little-endian word, zero above byte m:
-// one or two loads of the aligned words that hold them, shifted together.
-// Every such word holds at least one of the bytes, so it lies in the same
-// allocation (string heaps start 256-byte aligned and are padded at the end).
+// three aligned 32-bit loads and two funnel shifts.  They reach at most 8 bytes
+// past the string, inside its heap's allocation (heaps start 256-byte aligned
+// and have 256 bytes of padding behind them).
 __device__ __forceinline__ uint64_t load_bytes(const uint8_t* p, int m) {
   const unsigned long long at = (unsigned long long)p;
-  const unsigned long long* a = reinterpret_cast<const unsigned long long*>(at & ~7ull);
-  const int sh = (int)(at & 7);
-  uint64_t w = __ldg(a) >> (8 * sh);
-  if (sh + m > 8) w |= __ldg(a + 1) << (64 - 8 * sh);
-  return m >= 8 ? w : (w & ((1ull << (8 * m)) - 1));
+  const uint32_t* a = reinterpret_cast<const uint32_t*>(at & ~3ull);
+  const uint32_t sh = ((uint32_t)at & 3u) * 8u;
+  const uint32_t x = __ldg(a), y = __ldg(a + 1), z = __ldg(a + 2);
+  return (uint64_t)low_bytes(__funnelshift_r(x, y, sh), m) | ((uint64_t)low_bytes(__funnelshift_r(y, z, sh), m - 4) << 32);
 }
 
 // First index in [from, to) of byte c in s, or -1.  Tests eight bytes at a
@@ -460,9 +466,40 @@ __device__ __forceinline__ uint64_t warp_sum64(uint64_t v) {
 // strings are equal exactly when their lengths and words are.
 constexpr int kStrShortWords = kStrCoopMin / 8;
 
-__device__ __forceinline__ void str_words_short(const uint8_t* p, int n, uint64_t* w) {
+// Aligned 32-bit loads (those that hold bytes of the string) and funnel shifts,
+// 16 bytes at a time: strings up to 16 bytes skip the second half.
+__device__ __forceinline__ void str_words_16(const uint8_t* p, int n, uint64_t* w) {
+  const unsigned long long at = (unsigned long long)p;
+  const uint32_t* a = reinterpret_cast<const uint32_t*>(at & ~3ull);
+  const int lead = (int)(at & 3);
+  const uint32_t sh = (uint32_t)lead * 8u;
+  uint32_t x[5];
 #pragma unroll
-  for (int i = 0; i < kStrShortWords; ++i) w[i] = 8 * i < n ? load_bytes(p + 8 * i, n - 8 * i < 8 ? n - 8 * i : 8) : 0ull;
+  for (int i = 0; i < 5; ++i) x[i] = 4 * i < n + lead ? __ldg(a + i) : 0u;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    w[i] = (uint64_t)low_bytes(__funnelshift_r(x[2 * i], x[2 * i + 1], sh), n - 8 * i) |
+           ((uint64_t)low_bytes(__funnelshift_r(x[2 * i + 1], x[2 * i + 2], sh), n - 8 * i - 4) << 32);
+}
+
+__device__ __forceinline__ void str_words_short(const uint8_t* p, int n, uint64_t* w) {
+  static_assert(kStrShortWords == 4, "two halves of 16 bytes");
+  str_words_16(p, n, w);
+  w[2] = w[3] = 0ull;
+  if (n > 16) str_words_16(p + 16, n - 16, w + 2);
+}
+
+// A 32-bit hash of a short string from its words (a multilinear hash: one
+// multiply-add a 32-bit word), for CTA-local tables that compare the strings.
+__device__ __forceinline__ uint32_t str_hash32_words(const uint64_t* w, int n) {
+  uint32_t h = (uint32_t)n * 0x9e3779b1u;
+  h += (uint32_t)w[0] * 0x85ebca77u + (uint32_t)(w[0] >> 32) * 0xc2b2ae3du;
+  h += (uint32_t)w[1] * 0x27d4eb2fu + (uint32_t)(w[1] >> 32) * 0x165667b1u;
+  if (n > 16) {
+    h += (uint32_t)w[2] * 0x9e3779b9u + (uint32_t)(w[2] >> 32) * 0x7feb352du;
+    h += (uint32_t)w[3] * 0x846ca68bu + (uint32_t)(w[3] >> 32) * 0x2c1b3c6du;
+  }
+  return h;
 }
 
 __device__ __forceinline__ uint64_t str_hash_words(const uint64_t* w, int n) {

@@ -48,7 +48,7 @@ constexpr int kPrivateMax = 68 * 1024;      // shared memory per-thread accumula
 constexpr int kPrivateSlots = 64;           // group slots beside them
 constexpr int kBlock = kThreads;
 constexpr int kWarpBuf = 64;                // rows one warp's divergence buffer holds
-constexpr int kStrSlotWords = 6;            // a CTA-local group slot's string: location, length, 4 words
+constexpr int kStrSlotWords = 6;            // a CTA-local group slot's string: 4 words, length, location
 
 const char* ct_name(int t) {
   switch (t) {
@@ -336,7 +336,9 @@ struct Gen {
   // name them, per key index) for the comparisons that follow.  All keys are
   // located first and the short ones hashed by their lanes with independent
   // loads, so the loads of several keys overlap; long ones go to the warp.
-  std::string str_key_hashes(int r, int list, int n, const std::string& act) {
+  // With `lazy` a short string's hash is left to full_tag (the CTA-local group
+  // table finds its slot by the 32-bit hash `cheap` names).
+  std::string str_key_hashes(int r, int list, int n, const std::string& act, bool lazy = false) {
     str_ptr.assign((size_t)std::max(n, 0), std::string());
     str_len.assign((size_t)std::max(n, 0), std::string());
     str_words.assign((size_t)std::max(n, 0), std::string());
@@ -358,7 +360,7 @@ struct Gen {
         L("uint64_t " + w + "[kStrShortWords] = {};");
         L("if (" + act + " && " + str_len[(size_t)i] + " <= kStrCoopMin) {");
         L("  str_words_short(" + str_ptr[(size_t)i] + ", " + str_len[(size_t)i] + ", " + w + ");");
-        L("  " + h + "[" + num(i) + "] = str_hash_words(" + w + ", " + str_len[(size_t)i] + ");");
+        if (!lazy) L("  " + h + "[" + num(i) + "] = str_hash_words(" + w + ", " + str_len[(size_t)i] + ");");
         L("}");
         str_words[(size_t)i] = w;
       }
@@ -371,21 +373,52 @@ struct Gen {
     return h;
   }
 
-  // CTA-local group slot of a key with strings: linear probing over ns slots
-  // of ltags; a claim publishes the key values (lkeys, for the flush) and,
-  // per string, its location, length and words (lstr: kStrSlotWords words)
-  // before the tag.  A row whose tag matches compares lengths and words (a
-  // string of at most kStrCoopMin bytes) or its bytes with the slot string's
-  // (a longer one), without locating the slot's string again.  s_ stays -1
-  // when the table is full or a claim stays unpublished past the wait limit
-  // (the caller aggregates into the global table).
-  void local_str_slot(int r, const std::string& k) {
+  // Declares full_tag_: the key's tag in the global table (key_tag_strh over
+  // the resource's keys; short strings are hashed here, from their words).
+  void full_tag(int r, const std::string& k, const std::string& sh) {
+    const DevRes& R = P.res[r];
+    L("auto full_tag_ = [&]() -> uint64_t {");
+    ++ind;
+    L("uint64_t th_ = 0x9e3779b97f4a7c15ull;");
+    for (int q = 0; q < R.nkeys; ++q) {
+      std::string v = k + "[" + num(q) + "]";
+      if (R.key_ctype[q] == DQ_STR)
+        v = "(" + str_len[(size_t)q] + " <= kStrCoopMin ? str_hash_words(" + str_words[(size_t)q] + ", " +
+            str_len[(size_t)q] + ") : " + sh + "[" + num(q) + "])";
+      L("th_ = fmix64(th_ ^ " + v + ") + 0x632be59bd9b4e019ull * " + num(q + 1) + "ull;");
+    }
+    L("return fmix64(th_) & 0x7fffffffffffffffull;");
+    --ind;
+    L("};");
+  }
+
+  // CTA-local group slot of a key with strings: linear probing over the ns
+  // slots of ltags, which hold a 32-bit hash of the key.  A claim publishes the
+  // key values (lkeys) and their global tag (lfull) for the flush and, per
+  // string, its words, length and location (lstr: kStrSlotWords words) before
+  // the slot's hash.  A row whose hash matches compares lengths and words (a
+  // string of at most kStrCoopMin bytes, two words a load) or its bytes with the
+  // slot string's (a longer one), without locating the slot's string again.  s_
+  // stays -1 when the table is full or a claim stays unpublished past the wait
+  // limit (the caller aggregates into the global table).
+  void local_str_slot(int r, const std::string& k, const std::string& sh) {
     const DevRes& R = P.res[r];
     const std::string NK = num(R.nkeys), NS = num(ns), NSTR = num(nstr_keys(R));
     L("int s_ = -1;");
     L("{");
     ++ind;
-    L("uint32_t i_ = slot_of(tag_, " + NS + "u);");
+    L("uint32_t ch_ = 0u;");
+    for (int q = 0; q < R.nkeys; ++q) {
+      const std::string kv = k + "[" + num(q) + "]", hv = sh + "[" + num(q) + "]", n = str_len[(size_t)q];
+      std::string v = "(uint32_t)" + kv + " * 0xcc9e2d51u + (uint32_t)(" + kv + " >> 32) * 0x1b873593u";
+      if (R.key_ctype[q] == DQ_STR)
+        v = "(" + n + " <= kStrCoopMin ? str_hash32_words(" + str_words[(size_t)q] + ", " + n + ") : (uint32_t)" + hv +
+            " ^ (uint32_t)(" + hv + " >> 32))";
+      L("ch_ = ch_ * 0x2545f491u + (" + v + ");");
+    }
+    L("ch_ ^= ch_ >> 15;");
+    L("const uint64_t lt_ = ch_;");
+    L("uint32_t i_ = __umulhi(ch_ * 0x9e3779b1u, " + NS + "u);");
     L("for (int n_ = 0; n_ < " + NS + "; ++n_) {");
     ++ind;
     L("uint64_t t_ = ((volatile uint64_t*)ltags)[i_];");
@@ -398,14 +431,15 @@ struct Gen {
       L("((volatile uint64_t*)lkeys)[i_ * " + NK + " + " + num(q) + "] = " + k + "[" + num(q) + "];");
       if (R.key_ctype[q] != DQ_STR) continue;
       const std::string at = "((volatile uint64_t*)lstr)[(i_ * " + NSTR + " + " + num(j) + ") * " + num(kStrSlotWords);
-      L(at + "] = (uint64_t)" + str_ptr[(size_t)q] + ";");
-      L(at + " + 1] = (uint64_t)" + str_len[(size_t)q] + ";");
       for (int w = 0; w < kStrSlotWords - 2; ++w)
-        L(at + " + " + num(2 + w) + "] = " + str_words[(size_t)q] + "[" + num(w) + "];");
+        L(at + " + " + num(w) + "] = " + str_words[(size_t)q] + "[" + num(w) + "];");
+      L(at + " + 4] = (uint64_t)" + str_len[(size_t)q] + ";");
+      L(at + " + 5] = (uint64_t)" + str_ptr[(size_t)q] + ";");
       ++j;
     }
+    L("((volatile uint64_t*)lfull)[i_] = full_tag_();");
     L("__threadfence_block();");
-    L("((volatile uint64_t*)ltags)[i_] = tag_;");
+    L("((volatile uint64_t*)ltags)[i_] = lt_;");
     L("s_ = (int)i_;");
     L("break;");
     --ind;
@@ -415,26 +449,35 @@ struct Gen {
     L("}");
     L("for (long long w_ = 0; t_ == kBusy && w_ < kSpinLimit; ++w_) t_ = ((volatile uint64_t*)ltags)[i_];");
     L("if (t_ == kBusy) break;");
-    L("if (t_ == tag_) {");
+    L("if (t_ == lt_) {");
     ++ind;
     L("__threadfence_block();");
-    std::string eq;
+    L("bool eq_ = true;");
     for (int q = 0, j = 0; q < R.nkeys; ++q) {
-      if (!eq.empty()) eq += " && ";
       if (R.key_ctype[q] != DQ_STR) {
-        eq += "((volatile uint64_t*)lkeys)[i_ * " + NK + " + " + num(q) + "] == " + k + "[" + num(q) + "]";
+        L("eq_ = eq_ && ((volatile uint64_t*)lkeys)[i_ * " + NK + " + " + num(q) + "] == " + k + "[" + num(q) + "];");
         continue;
       }
-      const std::string at = "((volatile uint64_t*)lstr)[(i_ * " + NSTR + " + " + num(j) + ") * " + num(kStrSlotWords);
+      const std::string at = "reinterpret_cast<const ulonglong2*>(lstr + (i_ * " + NSTR + " + " + num(j) + ") * " +
+                             num(kStrSlotWords) + ")";
       const std::string& n = str_len[(size_t)q];
-      std::string words;
-      for (int w = 0; w < kStrSlotWords - 2; ++w)
-        words += (w ? " && " : "") + at + " + " + num(2 + w) + "] == " + str_words[(size_t)q] + "[" + num(w) + "]";
-      eq += "(int)" + at + " + 1] == " + n + " && (" + n + " <= kStrCoopMin ? (" + words +
-            ") : str_eq((const uint8_t*)" + at + "], " + n + ", " + str_ptr[(size_t)q] + ", " + n + "))";
+      const std::string& w = str_words[(size_t)q];
+      L("{");
+      L("  const ulonglong2 a_ = " + at + "[0], c_ = " + at + "[2];");
+      L("  eq_ = eq_ && (int)c_.x == " + n + ";");
+      L("  if (" + n + " <= kStrCoopMin) {");
+      L("    eq_ = eq_ && a_.x == " + w + "[0] && a_.y == " + w + "[1];");
+      L("    if (eq_ && " + n + " > 16) {");
+      L("      const ulonglong2 b_ = " + at + "[1];");
+      L("      eq_ = b_.x == " + w + "[2] && b_.y == " + w + "[3];");
+      L("    }");
+      L("  } else if (eq_) {");
+      L("    eq_ = str_eq((const uint8_t*)c_.y, " + n + ", " + str_ptr[(size_t)q] + ", " + n + ");");
+      L("  }");
+      L("}");
       ++j;
     }
-    L("if (" + eq + ") {");
+    L("if (eq_) {");
     L("  s_ = (int)i_;");
     L("  break;");
     L("}");
@@ -1204,6 +1247,21 @@ struct Gen {
   }
 
   // ---------------------------------------------------------------- sinks --
+  // Whether any op hashes or compares string keys.
+  bool string_keys() const {
+    for (int k = 0; k < P.nops; ++k)
+      switch (P.ops[k].kind) {
+        case DQ_OP_PROBE:
+        case DQ_OP_EXISTS:
+        case DQ_OP_AGG:
+        case DQ_OP_BUILD:
+        case DQ_OP_MM_COUNT:
+        case DQ_OP_MM_SCATTER:
+          if (has_str_key(P.res[P.ops[k].res])) return true;
+      }
+    return false;
+  }
+
   static bool has_str_key(const DevRes& R) {
     for (int i = 0; i < R.nkeys; ++i)
       if (R.key_ctype[i] == DQ_STR) return true;
@@ -1225,18 +1283,15 @@ struct Gen {
       L("}");
       return;
     }
-    const std::string sh = str_key_hashes(r, op.list, op.nlist, act);
+    const bool local_str = has_str_key(R) && agg != AGG_GLOBAL;
+    const std::string sh = str_key_hashes(r, op.list, op.nlist, act, has_str_key(R));
     L("if (" + act + ") {");
     ++ind;
     std::string k = keys(op, r, op.list, op.nlist);
     if (R.packed) L("const uint64_t tag_ = " + packed_tag(r, op.list, op.nlist) + ";");
     else if (has_str_key(R)) {
-      // key_tag_strh unrolled over the resource's keys
-      L("uint64_t th_ = 0x9e3779b97f4a7c15ull;");
-      for (int q = 0; q < R.nkeys; ++q)
-        L("th_ = fmix64(th_ ^ " + (R.key_ctype[q] == DQ_STR ? sh : k) + "[" + num(q) + "]) + 0x632be59bd9b4e019ull * " +
-          num(q + 1) + "ull;");
-      L("const uint64_t tag_ = fmix64(th_) & 0x7fffffffffffffffull;");
+      full_tag(r, k, sh);
+      if (!local_str) L("const uint64_t tag_ = full_tag_();");
     } else {
       L("const uint64_t tag_ = key_tag(" + res(r) + ", " + k + ");");
     }
@@ -1244,7 +1299,7 @@ struct Gen {
       if (R.packed) {
         packed_claim(r, "tag_");
       } else {
-        L("const int64_t g_ = agg_slot_global(P, " + res(r) + ", tag_, " + k + ");");
+        L("const int64_t g_ = agg_slot_global(P, " + res(r) + ", " + (local_str ? "full_tag_()" : "tag_") + ", " + k + ");");
       }
       L("if (g_ >= 0) {");
       ++ind;
@@ -1263,7 +1318,7 @@ struct Gen {
         L("const int s_ = local_group_slot_id(ltags, lids, lids + " + num(ns + 1) + ", " + num(ns) + ", " + num(shift) +
           ", tag_);");
       } else if (R.packed) L("const int s_ = local_group_slot(ltags, " + num(ns) + ", tag_, " + num(R.nkeys) + ");");
-      else if (has_str_key(R)) local_str_slot(r, k);
+      else if (has_str_key(R)) local_str_slot(r, k, sh);
       else L("const int s_ = local_group_slot_keys(P, " + res(r) + ", ltags, lkeys, " + num(ns) + ", tag_, " + k + ");");
       if (agg == AGG_PRIVATE) {
         // the group's accumulators of this thread: no other thread touches them
@@ -1511,7 +1566,7 @@ struct Gen {
     // twice as slow at five CTAs per SM as an 8.8 KB one), and even without
     // probes 32 copies of C0's table (26 KB) ran 8 % slower than 8 (6.5 KB)
     // hashed keys: their values too, and each string's location
-    const int tags = (ns + 1) * 8 + (R.packed ? 0 : ns * (R.nkeys + kStrSlotWords * nstr_keys(R)) * 8);
+    const int tags = (ns + 1) * 8 + (R.packed ? 0 : ns * (1 + R.nkeys + kStrSlotWords * nstr_keys(R)) * 8);
     agg = AGG_LOCAL;
     copies = 1;
     for (int c : {32, 16, 8, 4})
@@ -1729,17 +1784,15 @@ struct Gen {
         L("uint64_t acc" + num(j) + " = red_init(" + red_name(R.agg_red[j]) + ");");
       return;
     }
-    L("uint64_t* ltags = reinterpret_cast<uint64_t*>(smem);");
     if (R.packed) {
+      L("uint64_t* ltags = reinterpret_cast<uint64_t*>(smem);");
       L("uint64_t* lacc = ltags + " + num(ns + 1) + ";");
-    } else {
-      L("uint64_t* lkeys = ltags + " + num(ns + 1) + ";");
-      if (has_str_key(R)) {
-        L("uint64_t* lstr = lkeys + " + num(ns * R.nkeys) + ";");
-        L("uint64_t* lacc = lstr + " + num(ns * kStrSlotWords * nstr_keys(R)) + ";");
-      } else {
-        L("uint64_t* lacc = lkeys + " + num(ns * R.nkeys) + ";");
-      }
+    } else {  // string keys (hashed keys without strings have no CTA-local table); lstr 16-byte aligned
+      L("uint64_t* lstr = reinterpret_cast<uint64_t*>(smem);");
+      L("uint64_t* lkeys = lstr + " + num(ns * kStrSlotWords * nstr_keys(R)) + ";");
+      L("uint64_t* lfull = lkeys + " + num(ns * R.nkeys) + ";");
+      L("uint64_t* ltags = lfull + " + num(ns) + ";");
+      L("uint64_t* lacc = ltags + " + num(ns + 1) + ";");
     }
     L("for (int i = tid; i <= " + num(ns) + "; i += " + num(block) + ") ltags[i] = kEmpty;");
     L("for (int i = tid; i < " + num((ns + 1) * R.naggs * copies) + "; i += " + num(block) + ")");
@@ -1822,7 +1875,7 @@ struct Gen {
     if (copies > 1) L("for (int c_ = 1; c_ < " + num(copies) + "; ++c_) v_ = red_combine(red_, v_, lacc[i * " +
                       num(copies) + " + c_]);");
     if (R.packed) packed_claim(agg_res, "tg_");
-    else L("const int64_t g_ = agg_slot_global(P, " + rr + ", tg_, lkeys + s_ * " + num(R.nkeys) + ");");
+    else L("const int64_t g_ = agg_slot_global(P, " + rr + ", lfull[s_], lkeys + s_ * " + num(R.nkeys) + ");");
     L("if (g_ >= 0) accumulate(" + rr + ".slots + (uint64_t)g_ * " + num(R.words) + " + " + num(R.val_word) +
       " + j_, red_, v_);");
     --ind;
@@ -2357,6 +2410,11 @@ Program generate(const DevPipe& P, int expand_op, int refill_op, const Tuning& t
   bool scans = false;
   for (int k = 0; k < P.nops; ++k) scans |= g.scan_literal(k) >= 0;
   if (scans) g.U = 1;
+  // string keys: a row waits for its strings' offsets, then for their bytes, so
+  // more warps hide more of that than more rows a thread, whose registers the
+  // strings' words multiply (6 M rows grouped by two strings: one row a thread
+  // 184 us at 80 registers, two 225 us at 116, four 323 us at 120)
+  if (rows <= 0 && g.string_keys()) g.U = 1;
   g.choose_agg();
   g.choose_refill(refill_op);
   g.choose_hot();
