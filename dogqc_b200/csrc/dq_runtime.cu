@@ -334,7 +334,6 @@ struct PipeRec {
   int staged_cols = 0;
   int tail = -1;            // the pipeline this kernel's last CTA runs (fused tail)
   int fused_into = -1;      // runs inside that pipeline's kernel, not launched
-  DevBuf tail_buf;          // device copy of the fused tail's descriptor
 };
 
 struct dq_result {
@@ -1647,19 +1646,6 @@ void refresh_pipelines(dq_plan* plan) {
   for (auto& pp : plan->pipes) {
     pp->dev.strsrc = plan->str_src_dev.as<DevStr>();
     pp->dev.nstrsrc = (int32_t)n;
-  }
-  // fused tails: their descriptors where the kernels that run them read them
-  // (they always reset the aggregation table they scan: they are its only scan)
-  for (size_t i = 0; i < plan->pipes.size(); ++i) {
-    PipeRec& p = *plan->pipes[i];
-    if (p.tail < 0) continue;
-    PipeRec& t = *plan->pipes[p.tail];
-    t.dev.clear_src = 1;
-    t.dev.tile_counter = plan->counters + 2 * p.tail;
-    if (!p.tail_buf.ptr || p.tail_buf.bytes != sizeof(DevPipe)) p.tail_buf.alloc(sizeof(DevPipe));
-    if (!plan->ctx->offline && !t_offline)
-      DQ_CUDA(cudaMemcpy(p.tail_buf.ptr, &t.dev, sizeof(DevPipe), cudaMemcpyHostToDevice));
-    p.dev.tail = p.tail_buf.as<DevPipe>();
   }
 }
 
