@@ -964,15 +964,15 @@ __device__ __forceinline__ int local_group_slot_keys(const DevPipe& P, const Dev
 }
 
 // CTA-local table of multimap buckets (the hot buckets of a skewed build side
-// land in it first): kHotSlots bucket ids, kEmpty32 when free.  Returns the
-// bucket's slot, claiming a free one in its window of kHotProbe slots, or -1.
-
-__device__ __forceinline__ int hot_slot(uint32_t* keys, uint32_t b) {
+// land in it): kHotSlots bucket ids, kEmpty32 when free.  Returns the bucket's
+// slot in its window of kHotProbe slots, claiming a free one if `claim`, or -1.
+__device__ __forceinline__ int hot_slot(uint32_t* keys, uint32_t b, bool claim) {
   uint32_t idx = __umulhi(b * 0x9E3779B1u, (uint32_t)kHotSlots);
   for (int n = 0; n < kHotProbe; ++n) {
     const uint32_t k = ((volatile uint32_t*)keys)[idx];
     if (k == b) return (int)idx;
     if (k == kEmpty32) {
+      if (!claim) return -1;
       const uint32_t old = atomicCAS(&keys[idx], kEmpty32, b);
       if (old == kEmpty32 || old == b) return (int)idx;
     }

@@ -98,7 +98,15 @@ struct DevRes {
   uint64_t cap;           // slots (UNIQUE/AGG), buckets (MULTI), rows (OUTPUT)
   uint64_t* slots;        // UNIQUE/AGG: cap+1 slots (last = tag ~0 key)
   uint32_t* counts;       // MULTI
-  uint32_t* offsets;      // MULTI (cap+1)
+  uint64_t* ranges;       // MULTI (cap+1): a bucket's rows << 32 | its first payload row
+                          // (behind the last bucket: the rows of all)
+  uint32_t* rank;         // MULTI, ranked: a source row's rank in its bucket, left by
+                          // the count pass for the scatter pass (by source row)
+  int32_t ranked;
+  int32_t row_bytes;      // MULTI: > 0: a row's payload is one aligned item of that
+                          // size (field j at pay_off[j]), else a column per field
+  uint64_t pay_rows;      // MULTI: payload rows there is room for
+  int8_t pay_off[DQ_MAX_PAY];
   int32_t npay;
   int32_t naggs;
   int8_t pay_ctype[DQ_MAX_PAY];
@@ -257,10 +265,12 @@ struct ResultPack {
 
 struct BatchScanSeg {     // one multimap's bucket counts -> offsets
   uint32_t* counts;
-  uint32_t* offsets;
+  uint64_t* ranges;
   uint64_t n;             // buckets
   uint64_t block0;        // first scan block of this segment
   uint64_t nblocks;
+  int32_t ranked;         // the counts stay (a ranked multimap's scatter needs none)
+  int32_t pad;
 };
 
 struct BatchPack {        // one output column of one instance

@@ -190,8 +190,9 @@ struct Gen {
   int refill_threshold = 32;     // buffered rows that make the warp process them
   int nbuf = 0;                  // values per row in the warp buffers
   int buf_off = 0;               // shared-memory offset of the warp buffers
-  int hot = 0;                   // multimap sink through the CTA's hot-bucket table:
-                                 // 1 count (flushed at the end), 2 scatter (per step)
+  bool hot = false;              // ranked multimap count through the CTA's hot-bucket table
+  bool steps = false;            // ranked multimap pass that handles a thread's rows of a step together
+  std::map<int, std::string> item;  // multimap -> the gathered payload item of the current match
   int hot_off = 0;               // shared-memory offset of that table
   std::string inst_expr = "0u";  // the instance a deferred item belongs to (batches)
   std::string ldfn = "__ldcs";   // load function of streamed source columns
@@ -1035,13 +1036,91 @@ struct Gen {
     return false;
   }
 
+  // Whether ops k.. need a level-0 row's index: strings read in place, or the
+  // ranks of a multimap's source rows.
+  bool reads_row_after(int k) {
+    const dq_op& sink = P.ops[P.nops - 1];
+    return reads_strings_after(k) ||
+           ((sink.kind == DQ_OP_MM_COUNT || sink.kind == DQ_OP_MM_SCATTER) && P.res[sink.res].ranked);
+  }
+
   // gathers of level `lv` (the key columns first), key check, rest of the ops
   // Loads a gathered multimap payload value of match `m` for the active lanes.
   void gather(int s, const std::string& act, const std::string& m) {
     const DevSlot& g = slot(s);
+    const DevRes& R = P.res[g.res];
     var[s] = "v" + num(s) + "_" + num(uid++);
+    auto it = item.find(g.res);
+    if (it != item.end()) {  // a field of the match's payload item
+      const int o = R.pay_off[g.src], w = g.width;
+      auto word = [&](int k) { return it->second + (R.row_bytes == 4 ? std::string() : std::string(".") + "xyzw"[k]); };
+      std::string v;
+      if (w == 8) v = "((uint64_t)" + word(o / 4) + " | ((uint64_t)" + word(o / 4 + 1) + " << 32))";
+      else if (w == 4) v = "(uint64_t)" + word(o / 4);
+      else v = "(uint64_t)((" + word(o / 4) + " >> " + num(8 * (o % 4)) + ") & " + (w == 2 ? "0xffffu" : "0xffu") + ")";
+      L("const uint64_t " + var[s] + " = canon(" + v + ", " + ct_name(g.ctype) + ");");
+      return;
+    }
     L("const uint64_t " + var[s] + " = " + act + " ? canon(ldg_w(" + res(g.res) + ".pay[" + num(g.src) +
-      "] + (uint64_t)" + m + " * " + num(g.width) + ", " + num(g.width) + "), " + ct_name(g.ctype) + ") : 0ull;");
+      "] + (uint64_t)" + m + " * " + num(R.row_bytes > 0 ? R.row_bytes : g.width) + ", " + num(g.width) + "), " +
+      ct_name(g.ctype) + ") : 0ull;");
+  }
+
+  static const char* item_type(int bytes) { return bytes == 16 ? "uint4" : bytes == 8 ? "uint2" : "uint32_t"; }
+
+  // Loads the payload item of match `m` of multimap r (one load) when its rows
+  // are items; gather() then takes its fields.
+  void gather_item(int r, const std::string& act, const std::string& m) {
+    const DevRes& R = P.res[r];
+    if (R.row_bytes <= 0 || R.npay <= 0) return;
+    const std::string T = item_type(R.row_bytes), v = fresh("gi");
+    L(T + " " + v + " = " + (R.row_bytes == 16 ? "make_uint4(0u, 0u, 0u, 0u)" : R.row_bytes == 8 ? "make_uint2(0u, 0u)" : "0u") + ";");
+    L("if (" + act + ") " + v + " = reinterpret_cast<const " + T + "*>(" + res(r) + ".pay[" + num(item_base(r)) + "])[" + m + "];");
+    item[r] = v;
+  }
+
+  // The field at an item's start.
+  int item_base(int r) const {
+    for (int j = 0; j < P.res[r].npay; ++j)
+      if (P.res[r].pay_off[j] == 0) return j;
+    throw Error("payload item without a first field");
+  }
+
+  // Stores the payload values (canonical, in `v`) as row `pos` of multimap r.
+  void store_payload(int r, const std::string& pos, const std::vector<std::string>& v) {
+    const DevRes& R = P.res[r];
+    if (v.empty()) return;
+    L("if (" + pos + " >= " + res(r) + ".pay_rows) {  // more rows than were there at preparation");
+    L("  set_status(P, kErrOverflow);");
+    L("} else {");
+    ++ind;
+    if (R.row_bytes > 0) {
+      std::vector<std::string> word((size_t)R.row_bytes / 4);
+      auto put = [&](int k, const std::string& x) { word[(size_t)k] += (word[(size_t)k].empty() ? "" : " | ") + x; };
+      for (size_t j = 0; j < v.size(); ++j) {
+        const int o = R.pay_off[j], w = R.pay_width[j];
+        if (w == 8) {
+          put(o / 4, "(uint32_t)(" + v[j] + ")");
+          put(o / 4 + 1, "(uint32_t)((" + v[j] + ") >> 32)");
+        } else if (w == 4) {
+          put(o / 4, "(uint32_t)(" + v[j] + ")");
+        } else {
+          put(o / 4, "((uint32_t)(" + v[j] + ") & " + (w == 2 ? "0xffffu" : "0xffu") + ") << " + num(8 * (o % 4)));
+        }
+      }
+      std::string all;
+      for (auto& w : word) all += (all.empty() ? "" : ", ") + (w.empty() ? std::string("0u") : w);
+      const std::string T = item_type(R.row_bytes);
+      L("reinterpret_cast<" + T + "*>(" + res(r) + ".pay[" + num(item_base(r)) + "])[" + pos + "] = " +
+        (R.row_bytes == 4 ? all : "make_" + T + "(" + all + ")") + ";");
+    } else {
+      for (size_t j = 0; j < v.size(); ++j) {
+        const int w = R.pay_width[j];
+        L("st(" + res(r) + ".pay[" + num((long long)j) + "] + (size_t)" + pos + " * " + num(w) + ", " + num(w) + ", " + v[j] + ");");
+      }
+    }
+    --ind;
+    L("}");
   }
 
   // Gathers the pending payload values the given slots need (lanes that a
@@ -1069,6 +1148,8 @@ struct Gen {
   // The payload values of level `lv` for match `m` (the key columns first).
   void gather_level(int k, int lv, const std::string& a, const std::string& m) {
     const dq_op& op = P.ops[k];
+    item.clear();
+    gather_item(op.res, a, m);
     for (int q = 0; q < op.nlist2; ++q) {
       int s = P.lists[op.list2 + q];
       if (s >= 0 && slot(s).kind == DQ_SLOT_GATHER && slot(s).level == lv && var[s].empty()) gather(s, a, m);
@@ -1110,12 +1191,15 @@ struct Gen {
     ++ind;
     std::string kk = keys(op, r, op.list, op.nlist);
     L("const uint32_t b_ = " + bucket(op, r, kk, sh) + ";");
-    L("const uint32_t xc_ = " + res(r) + ".counts[b_];");
-    L("uint32_t " + m + " = xc_ ? " + res(r) + ".offsets[b_] : 0u;");
-    L("const uint32_t " + me + " = " + m + " + xc_;");
+    L("const uint64_t xr_ = " + res(r) + ".ranges[b_];");
+    L("uint32_t " + m + " = (uint32_t)xr_;");
+    L("const uint32_t " + me + " = " + m + " + (uint32_t)(xr_ >> 32);");
     L("for (; " + m + " < " + me + "; ++" + m + ") {");
     ++ind;
     const std::vector<std::string> saved = var;
+    const std::map<int, std::string> saved_item = item;
+    item.clear();
+    gather_item(r, "true", m);
     for (int s2 = 0; s2 < P.nslots; ++s2)
       if (slot(s2).kind == DQ_SLOT_GATHER && slot(s2).level == lv && slot(s2).res == r) gather(s2, "true", m);
     std::string eq = "true";
@@ -1129,6 +1213,7 @@ struct Gen {
     L(fm + " = true;");
     L("break;");
     var = saved;  // the build row's values end with the walk
+    item = saved_item;
     --ind;
     L("}");
     --ind;
@@ -1150,8 +1235,9 @@ struct Gen {
     ++ind;
     std::string kk = keys(op, r, op.list, op.nlist);
     L("const uint32_t b_ = " + bucket(op, r, kk, sh) + ";");
-    L(ec + " = " + res(r) + ".counts[b_];");
-    L(eo + " = " + ec + " ? " + res(r) + ".offsets[b_] : 0u;");
+    L("const uint64_t xr_ = " + res(r) + ".ranges[b_];");
+    L(eo + " = (uint32_t)xr_;");
+    L(ec + " = (uint32_t)(xr_ >> 32);");
     --ind;
     L("}");
     if (k == expand_op && level == 0) {
@@ -1409,12 +1495,16 @@ struct Gen {
     L("}");
   }
 
+  // A ranked multimap's count pass leaves every source row's rank in its
+  // bucket for the scatter pass, which then needs no second round of atomics:
+  // a row's place is its bucket's offset plus its rank.  (6 M rows over 3 M
+  // buckets, both passes and the scan: 237 -> 190 us.)  Lanes of a warp that hit the same
+  // bucket (the hot keys of a skewed build side) take one atomic per bucket: the
+  // lowest such lane adds the group's size, the others their rank in it.
   void sink_mm(const dq_op& op, const std::string& act) {
-    // lanes of a warp that hit the same bucket (the hot keys of a skewed build
-    // side) take one atomic per bucket: the lowest such lane adds the group's
-    // size, the others their rank within the group
     const int r = op.res;
     const DevRes& R = P.res[r];
+    const bool scatter = op.kind == DQ_OP_MM_SCATTER;
     const std::string sh = str_key_hashes(r, op.list, op.nlist, act);
     L("uint32_t b_ = 0xffffffffu;");
     L("if (" + act + ") {");
@@ -1423,56 +1513,51 @@ struct Gen {
     L("b_ = " + bucket(op, r, k, sh) + ";");
     --ind;
     L("}");
+    std::vector<std::string> vals;
+    if (scatter)
+      for (int j = 0; j < op.nlist2; ++j) vals.push_back(V(P.lists[op.list2 + j]));
+    if (R.ranked && scatter) {
+      if (steps) {  // placed at the end of the step, when the offsets of all rows are on their way
+        L("if (" + act + ") {");
+        ++ind;
+        L("po_u[u] = (uint32_t)" + res(r) + ".ranges[b_];");
+        L("pa_u |= 1u << u;");
+        for (int j = 0; j < op.nlist2; ++j)
+          if (step_value(op, j, "u").empty()) L("hv" + num(j) + "_u[u] = " + vals[(size_t)j] + ";");
+        --ind;
+        L("}");
+      } else {
+        L("if (" + act + ") {");
+        ++ind;
+        L("const uint32_t pos_ = (uint32_t)" + res(r) + ".ranges[b_] + " + res(r) + ".rank[" + row + "];");
+        store_payload(r, "pos_", vals);
+        --ind;
+        L("}");
+      }
+      return;
+    }
+    if (R.ranked && steps) {  // counted at the end of the step
+      L("bk_u[u] = b_;");
+      return;
+    }
     L("const unsigned peers_ = __match_any_sync(kFull, b_);");
     L("if (" + act + ") {");
     ++ind;
     L("const int lead_ = __ffs(peers_) - 1;");
-    if (hot == 1) {
-      L("if (lane == lead_) {");
-      L("  const int hs_ = hot_slot(hk_, b_);");
-      L("  if (hs_ >= 0) atomicAdd(&hc_[hs_], (uint32_t)__popc(peers_));");
-      L("  else atomicAdd(&" + res(r) + ".counts[b_], (uint32_t)__popc(peers_));");
-      L("}");
-    } else if (hot == 2) {
-      // the bucket's offset does not depend on the claim: load it first
-      L("const uint32_t ob_ = " + res(r) + ".offsets[b_];");
-      L("int hs_ = -1;");
+    L("const int np_ = __popc(peers_);");
+    if (R.ranked) {
       L("uint32_t at_ = 0;");
-      L("if (lane == lead_) {");
-      L("  hs_ = hot_slot(hk_, b_);");
-      L("  at_ = atomicAdd(hs_ >= 0 ? &hc_[hs_] : &" + res(r) + ".counts[b_], (uint32_t)__popc(peers_));");
-      L("}");
-      L("hs_ = __shfl_sync(peers_, hs_, lead_);");
+      L("if (lane == lead_) at_ = atomicAdd(&" + res(r) + ".counts[b_], (uint32_t)np_);");
       L("at_ = __shfl_sync(peers_, at_, lead_) + (uint32_t)__popc(peers_ & ((1u << lane) - 1u));");
-      L("if (hs_ >= 0) {");
-      ++ind;
-      L("hs_u[u] = hs_;");
-      L("hr_u[u] = ob_ + at_;");
-      for (int j = 0; j < op.nlist2; ++j)
-        if (hot_value(op, j, "u").empty()) L("hv" + num(j) + "_u[u] = " + V(P.lists[op.list2 + j]) + ";");
-      --ind;
-      L("} else {");
-      ++ind;
-      L("const uint32_t pos_ = ob_ + at_;");
-      for (int j = 0; j < op.nlist2; ++j) {
-        int w = R.pay_width[j];
-        L("st(" + res(r) + ".pay[" + num(j) + "] + (size_t)pos_ * " + num(w) + ", " + num(w) + ", " +
-          V(P.lists[op.list2 + j]) + ");");
-      }
-      --ind;
-      L("}");
-    } else if (op.kind == DQ_OP_MM_COUNT) {
-      L("if (lane == lead_) atomicAdd(&" + res(r) + ".counts[b_], (uint32_t)__popc(peers_));");
+      L(res(r) + ".rank[" + row + "] = at_;");
+    } else if (!scatter) {
+      L("if (lane == lead_) atomicAdd(&" + res(r) + ".counts[b_], (uint32_t)np_);");
     } else {
       L("uint32_t at_ = 0;");
-      L("if (lane == lead_) at_ = atomicAdd(&" + res(r) + ".counts[b_], (uint32_t)__popc(peers_));");
+      L("if (lane == lead_) at_ = atomicAdd(&" + res(r) + ".counts[b_], (uint32_t)np_);");
       L("at_ = __shfl_sync(peers_, at_, lead_);");
-      L("const uint32_t pos_ = " + res(r) + ".offsets[b_] + at_ + (uint32_t)__popc(peers_ & ((1u << lane) - 1u));");
-      for (int j = 0; j < op.nlist2; ++j) {
-        int w = R.pay_width[j];
-        L("st(" + res(r) + ".pay[" + num(j) + "] + (size_t)pos_ * " + num(w) + ", " + num(w) + ", " +
-          V(P.lists[op.list2 + j]) + ");");
-      }
+      L("const uint32_t pos_ = (uint32_t)" + res(r) + ".ranges[b_] + at_ + (uint32_t)__popc(peers_ & ((1u << lane) - 1u));");
+      store_payload(r, "pos_", vals);
     }
     --ind;
     L("}");
@@ -1599,27 +1684,28 @@ struct Gen {
     }
     if (!heavy) return;
     refill = k;
-    nbuf = (int)live_after(k + 1, 0).size() + (reads_strings_after(k + 1) ? 1 : 0);
+    nbuf = (int)live_after(k + 1, 0).size() + (reads_row_after(k + 1) ? 1 : 0);
     if (nbuf == 0) nbuf = 1;
     buf_off = (smem + 15) / 16 * 16;
     smem = buf_off + (block / 32) * kWarpBuf * nbuf * 8;
   }
 
-  // Multimap sinks of a skewed build side meet on a few buckets: a CTA-local
-  // table of buckets takes their counts (count pass) or ranks (scatter pass),
-  // so a hot bucket sees one global atomic per CTA (count) or per CTA and row
-  // step (scatter) instead of one per warp.  The scatter pass reserves ranges
-  // at the end of every row step behind block barriers, so it needs straight
-  // row steps: no lane refill, no expansion.
+  // Multimap builds of a skewed build side meet on a few buckets: in the count
+  // pass a CTA-local table of buckets takes their ranks, so a hot bucket sees
+  // one global atomic per CTA and row step instead of one per warp.  Ranges are
+  // reserved at the end of every row step behind block barriers, so that needs
+  // straight row steps: no lane refill.  Both ranked passes then handle a
+  // thread's rows of a step together: the ranks are one vector store or load a
+  // thread, and the scatter's offset loads overlap.
   void choose_hot() {
-    hot = 0;
-    if (batched || P.nops == 0) return;
-    const int kind = P.ops[P.nops - 1].kind;
-    if (kind != DQ_OP_MM_COUNT && kind != DQ_OP_MM_SCATTER) return;
-    for (int j = 0; j < P.nops; ++j)
-      if (P.ops[j].kind == DQ_OP_EXPAND) return;
-    if (kind == DQ_OP_MM_SCATTER && refill >= 0) return;
-    hot = kind == DQ_OP_MM_COUNT ? 1 : 2;
+    hot = steps = false;
+    if (batched || P.nops == 0 || refill >= 0) return;
+    const dq_op& sink = P.ops[P.nops - 1];
+    if (sink.kind != DQ_OP_MM_COUNT && sink.kind != DQ_OP_MM_SCATTER) return;
+    if (!P.res[sink.res].ranked) return;
+    steps = true;
+    hot = sink.kind == DQ_OP_MM_COUNT;
+    if (!hot) return;
     hot_off = (smem + 15) / 16 * 16;
     smem = hot_off + kHotSlots * 12;
   }
@@ -1627,9 +1713,8 @@ struct Gen {
   void hot_init() {
     if (!hot) return;
     L("uint32_t* const hk_ = reinterpret_cast<uint32_t*>(smem + " + num(hot_off) + ");  // hot buckets");
-    L("uint32_t* const hc_ = hk_ + " + num(kHotSlots) + ";  // their counts (of this step when scattering)");
-    L("uint32_t* const hb_ = hc_ + " + num(kHotSlots) + ";  // their reserved range starts");
-    L("(void)hb_;");
+    L("uint32_t* const hc_ = hk_ + " + num(kHotSlots) + ";  // their rows in this step");
+    L("uint32_t* const hb_ = hc_ + " + num(kHotSlots) + ";  // their reserved ranks' starts");
     L("for (int i = tid; i < " + num(kHotSlots) + "; i += " + num(block) + ") {");
     L("  hk_[i] = kEmpty32;");
     L("  hc_[i] = 0u;");
@@ -1637,36 +1722,102 @@ struct Gen {
     L("__syncthreads();");
   }
 
-  // Scatter pass: per-row state of the table rows of the current step.
-  void hot_step_begin() {
-    if (hot != 2) return;
+  // A ranked pass's per-row state in the current step, and the ranks of the
+  // thread's rows (r0_ = base + tid * U, U consecutive ones).
+  void rank_step_begin() {
+    if (!steps) return;
     const dq_op& op = P.ops[P.nops - 1];
-    L("int hs_u[" + num(U) + "];");
-    L("uint32_t hr_u[" + num(U) + "];  // bucket offset + rank in the step");
+    const std::string Us = num(U), rank = res(op.res) + ".rank";
+    const char* T = U == 4 ? "uint4" : U == 2 ? "uint2" : "uint32_t";
+    if (op.kind == DQ_OP_MM_COUNT) {
+      L("uint32_t bk_u[" + Us + "];  // buckets of the thread's rows");
+      L("#pragma unroll");
+      L("for (int u = 0; u < " + Us + "; ++u) bk_u[u] = 0xffffffffu;");
+      return;
+    }
+    L("uint32_t rk_u[" + Us + "];");
+    L("uint32_t po_u[" + Us + "], pa_u = 0u;");
     for (int j = 0; j < op.nlist2; ++j)
-      if (hot_value(op, j, "u").empty()) L("uint64_t hv" + num(j) + "_u[" + num(U) + "];");
+      if (step_value(op, j, "u").empty()) L("uint64_t hv" + num(j) + "_u[" + Us + "];");
+    L("{");
+    ++ind;
+    L("const int64_t r0_ = base + (int64_t)tid * " + Us + ";");
+    L("if (r0_ + " + Us + " <= nrows) {");
+    L(std::string("  const ") + T + " x_ = __ldcs(reinterpret_cast<const " + T + "*>(" + rank + " + r0_));");
+    if (U == 1) L("  rk_u[0] = x_;");
+    for (int u = 0; u < U && U > 1; ++u) L("  rk_u[" + num(u) + "] = x_." + "xyzw"[u] + ";");
+    L("} else {");
     L("#pragma unroll");
-    L("for (int u = 0; u < " + num(U) + "; ++u) hs_u[u] = -1;");
+    L("  for (int u = 0; u < " + Us + "; ++u) rk_u[u] = r0_ + u < nrows ? " + rank + "[r0_ + u] : 0u;");
+    L("}");
+    --ind;
+    L("}");
   }
 
-  // Payload value j of a deferred table row in the scatter's last phase: a
-  // source column value is still in the step's column registers; anything else
-  // was kept in hv<j>_u (empty result).
-  std::string hot_value(const dq_op& op, int j, const std::string& u) {
+  // Payload value j of a row in the scatter's last phase: a source column value
+  // is still in the step's column registers; anything else was kept in hv<j>_u
+  // (empty result).
+  std::string step_value(const dq_op& op, int j, const std::string& u) {
     const int s = P.lists[op.list2 + j];
     if (s >= 0 && slot(s).kind == DQ_SLOT_COL)
       return "canon(c" + num(slot(s).src) + "[" + u + "], " + ct_name(slot(s).ctype) + ")";
     return std::string();
   }
 
-  // Scatter pass: one global range per hot bucket of the step, then the
-  // table rows' payload at range start + rank.
-  void hot_step_end() {
-    if (hot != 2) return;
+  void rank_step_end() {
+    if (!steps) return;
     const dq_op& op = P.ops[P.nops - 1];
     const int r = op.res;
-    const DevRes& R = P.res[r];
-    L("__syncthreads();");
+    const std::string Us = num(U), rank = res(r) + ".rank";
+    const char* T = U == 4 ? "uint4" : U == 2 ? "uint2" : "uint32_t";
+    if (op.kind == DQ_OP_MM_SCATTER) {
+      L("#pragma unroll");
+      L("for (int u = 0; u < " + Us + "; ++u) {");
+      ++ind;
+      L("if ((pa_u >> u) & 1u) {");
+      ++ind;
+      L("const uint32_t pos_ = po_u[u] + rk_u[u];");
+      std::vector<std::string> vals;
+      for (int j = 0; j < op.nlist2; ++j) {
+        std::string v = step_value(op, j, "u");
+        vals.push_back(v.empty() ? "hv" + num(j) + "_u[u]" : v);
+      }
+      store_payload(r, "pos_", vals);
+      --ind;
+      L("}");
+      --ind;
+      L("}");
+      return;
+    }
+    // the atomics of the thread's rows first, all in flight, then their results
+    L("uint32_t rk_u[" + Us + "];");
+    L("unsigned pe_u[" + Us + "];");
+    L("int hs_u[" + Us + "], met_ = 0;");
+    L("#pragma unroll");
+    L("for (int u = 0; u < " + Us + "; ++u) {");
+    ++ind;
+    L("const uint32_t b_ = bk_u[u];");
+    L("pe_u[u] = __match_any_sync(kFull, b_);");
+    L("hs_u[u] = -1;");
+    L("rk_u[u] = 0u;");
+    L("if (b_ != 0xffffffffu && lane == __ffs(pe_u[u]) - 1) {");
+    ++ind;
+    L("const int np_ = __popc(pe_u[u]);");
+    L("const int h_ = hot_slot(hk_, b_, np_ > 1);  // a bucket enters the table when a warp meets it twice");
+    L("if (h_ >= 0) {");
+    L("  rk_u[u] = atomicAdd(&hc_[h_], (uint32_t)np_);");
+    L("  hs_u[u] = h_;");
+    L("  met_ = 1;");
+    L("} else {");
+    L("  rk_u[u] = atomicAdd(&" + res(r) + ".counts[b_], (uint32_t)np_);");
+    L("}");
+    --ind;
+    L("}");
+    --ind;
+    L("}");
+    L("const int any_ = __syncthreads_or(met_);");
+    L("if (any_) {  // one global range per hot bucket of the step");
+    ++ind;
     L("for (int i = tid; i < " + num(kHotSlots) + "; i += " + num(block) + ") {");
     L("  const uint32_t c_ = hc_[i];");
     L("  if (c_) {");
@@ -1676,31 +1827,25 @@ struct Gen {
     L("}");
     L("__syncthreads();");
     L("#pragma unroll");
-    L("for (int u = 0; u < " + num(U) + "; ++u) {");
-    ++ind;
-    L("if (hs_u[u] >= 0) {");
-    ++ind;
-    L("const uint32_t pos_ = hb_[hs_u[u]] + hr_u[u];");
-    for (int j = 0; j < op.nlist2; ++j) {
-      int w = R.pay_width[j];
-      std::string v = hot_value(op, j, "u");
-      if (v.empty()) v = "hv" + num(j) + "_u[u]";
-      L("st(" + res(r) + ".pay[" + num(j) + "] + (size_t)pos_ * " + num(w) + ", " + num(w) + ", " + v + ");");
-    }
+    L("for (int u = 0; u < " + Us + "; ++u)");
+    L("  if (hs_u[u] >= 0) rk_u[u] += hb_[hs_u[u]];");
     --ind;
     L("}");
-    --ind;
+    L("#pragma unroll");
+    L("for (int u = 0; u < " + Us + "; ++u)");
+    L("  rk_u[u] = __shfl_sync(kFull, rk_u[u], __ffs(pe_u[u]) - 1) + (uint32_t)__popc(pe_u[u] & ((1u << lane) - 1u));");
+    L("{");
+    ++ind;
+    L("const int64_t r0_ = base + (int64_t)tid * " + Us + ";");
+    L("if (r0_ + " + Us + " <= nrows) {");
+    L(std::string("  *reinterpret_cast<") + T + "*>(" + rank + " + r0_) = " +
+      (U == 4 ? "make_uint4(rk_u[0], rk_u[1], rk_u[2], rk_u[3])" : U == 2 ? "make_uint2(rk_u[0], rk_u[1])" : "rk_u[0]") + ";");
+    L("} else {");
+    L("#pragma unroll");
+    L("  for (int u = 0; u < " + Us + "; ++u)");
+    L("    if (r0_ + u < nrows) " + rank + "[r0_ + u] = rk_u[u];");
     L("}");
-  }
-
-  // Count pass: the table's counts go to the global ones once per CTA.
-  void hot_flush() {
-    if (hot != 1) return;
-    const int r = P.ops[P.nops - 1].res;
-    L("__syncthreads();");
-    L("for (int i = tid; i < " + num(kHotSlots) + "; i += " + num(block) + ") {");
-    L("  const uint32_t c_ = hc_[i];");
-    L("  if (c_) atomicAdd(&" + res(r) + ".counts[hk_[i]], c_);");
+    --ind;
     L("}");
   }
 
@@ -1710,7 +1855,7 @@ struct Gen {
   // do-while, which it closes and reopens.
   void refill_lanes(int k, const std::string& act) {
     std::vector<int> live = live_after(k + 1, 0);
-    const bool need_row = reads_strings_after(k + 1);
+    const bool need_row = reads_row_after(k + 1);
     const std::string B = num(kWarpBuf);
     L("{");
     ++ind;
@@ -2112,9 +2257,9 @@ struct Gen {
         L("}");
       }
     }
-    hot_step_begin();
+    rank_step_begin();
     row_loop();
-    hot_step_end();
+    rank_step_end();
     if (!cols.empty()) {
       L("#pragma unroll");
       L("for (int u = 0; u < " + num(U) + "; ++u) {");
@@ -2123,7 +2268,6 @@ struct Gen {
     }
     --ind;
     L("}");
-    hot_flush();
     epilogue();
   }
 

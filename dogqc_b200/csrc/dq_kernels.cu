@@ -357,7 +357,7 @@ __device__ void op_mm(const DevPipe& P, const Cta& c, const dq_op& op, const Lev
     if (op.kind == DQ_OP_MM_COUNT) {
       atomicAdd(&R.counts[b], 1u);
     } else {
-      uint32_t pos = R.offsets[b] + atomicAdd(&R.counts[b], 1u);
+      uint32_t pos = (uint32_t)R.ranges[b] + atomicAdd(&R.counts[b], 1u);
       for (int j = 0; j < op.nlist2; ++j)
         st(R.pay[j] + (size_t)pos * R.pay_width[j], R.pay_width[j],
            read_slot(P, c, P.lists[op.list2 + j], L.level, row));
@@ -441,7 +441,7 @@ __device__ uint32_t expand_setup(const DevPipe& P, const Cta& c, const dq_op& op
     key_values(P, c, R, op.list, op.nlist, L.level, row, k);
     uint64_t b = bucket_of(k, op.nlist, (uint32_t)R.cap);
     uint32_t cnt = R.counts[b];
-    uint32_t off = cnt ? R.offsets[b] : 0;
+    uint32_t off = cnt ? (uint32_t)R.ranges[b] : 0;
     if (defer && cnt > P.heavy.threshold) {
       uint32_t slot = atomicAdd(P.heavy.count, 1u);
       if (slot < P.heavy.cap) {
@@ -1097,7 +1097,7 @@ __device__ void row_ops(Row& x, bool act, uint8_t* smem) {
           if (op.kind == DQ_OP_MM_COUNT) {
             atomicAdd(&R.counts[b], 1u);
           } else {
-            uint32_t pos = R.offsets[b] + atomicAdd(&R.counts[b], 1u);
+            uint32_t pos = (uint32_t)R.ranges[b] + atomicAdd(&R.counts[b], 1u);
             for (int j = 0; j < op.nlist2; ++j)
               st(R.pay[j] + (size_t)pos * R.pay_width[j], R.pay_width[j], rget(x, P.lists[op.list2 + j]));
           }
@@ -1207,7 +1207,10 @@ __global__ void __launch_bounds__(kThreads, 3) row_kernel(const __grid_constant_
 
 // ------------------------------------------------------- helper kernels --
 
-// Multimap bucket offsets: exclusive scan of counts in three passes.
+// Multimap bucket ranges: exclusive scan of counts in three passes.  A probe
+// reads its bucket's first row and row count in one 8-byte load: random loads
+// cost the SM's L1 a cycle a lane, which bounds the sparse probes (16.8 M rows:
+// 129 us with two loads, 115 with one).
 constexpr int kScanItems = 16;
 constexpr int kScanChunk = kThreads * kScanItems;
 
@@ -1249,10 +1252,11 @@ __global__ void mm_scan_top(uint32_t* partials, int nblocks) {
   }
 }
 
-// Offsets of one chunk of buckets (kScanItems consecutive counts a thread, in
-// 16-byte vectors when the chunk is whole) and the counts reset to zero for the
-// scatter pass that follows.
-__global__ void mm_scan_final(uint32_t* counts, uint32_t* offsets, uint64_t n, const uint32_t* partials) {
+// Ranges of one chunk of buckets (kScanItems consecutive counts a thread, in
+// 16-byte vectors when the chunk is whole), the total behind the last one, and
+// the counts reset to zero for a scatter pass that counts again (not a ranked
+// multimap's).
+__global__ void mm_scan_final(uint32_t* counts, uint64_t* ranges, uint64_t n, const uint32_t* partials, int ranked) {
   static_assert(kScanItems % 4 == 0, "vector path");
   const uint64_t i0 = (uint64_t)blockIdx.x * kScanChunk + (uint64_t)threadIdx.x * kScanItems;
   const bool whole = i0 + kScanItems <= n;
@@ -1279,27 +1283,27 @@ __global__ void mm_scan_final(uint32_t* counts, uint32_t* offsets, uint64_t n, c
   if (whole) {
 #pragma unroll
     for (int k = 0; k < kScanItems; k += 4) {
-      uint4 o;
-      o.x = run;
-      run += v[k];
-      o.y = run;
-      run += v[k + 1];
-      o.z = run;
-      run += v[k + 2];
-      o.w = run;
-      run += v[k + 3];
-      *reinterpret_cast<uint4*>(offsets + i0 + k) = o;
-      *reinterpret_cast<uint4*>(counts + i0 + k) = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int q = 0; q < 4; q += 2) {
+        ulonglong2 o;
+        o.x = (uint64_t)v[k + q] << 32 | run;
+        run += v[k + q];
+        o.y = (uint64_t)v[k + q + 1] << 32 | run;
+        run += v[k + q + 1];
+        *reinterpret_cast<ulonglong2*>(ranges + i0 + k + q) = o;
+      }
+      if (!ranked) *reinterpret_cast<uint4*>(counts + i0 + k) = make_uint4(0u, 0u, 0u, 0u);
     }
   } else {
     for (int k = 0; k < kScanItems; ++k) {
       if (i0 + k < n) {
-        offsets[i0 + k] = run;
-        counts[i0 + k] = 0;
+        ranges[i0 + k] = (uint64_t)v[k] << 32 | run;
+        if (!ranked) counts[i0 + k] = 0;
       }
       run += v[k];
     }
   }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kThreads - 1) ranges[n] = run;
 }
 
 // Work-unit prefix over deferred expansion items (one block).
@@ -1601,11 +1605,12 @@ __global__ void batch_scan_final(const BatchScanSeg* segs, int nseg, const uint3
   uint32_t run = partials[b] + excl;
   for (int k = 0; k < kScanItems; ++k) {
     if (i0 + k < s.n) {
-      s.offsets[i0 + k] = run;
-      s.counts[i0 + k] = 0;
+      s.ranges[i0 + k] = (uint64_t)v[k] << 32 | run;
+      if (!s.ranked) s.counts[i0 + k] = 0;
     }
     run += v[k];
   }
+  if (b == s.block0 + s.nblocks - 1 && threadIdx.x == kThreads - 1) s.ranges[s.n] = run;
 }
 
 // Copies every instance's output columns (the rows emitted, at most the
@@ -1658,13 +1663,13 @@ int pipeline_occupancy(int smem_bytes) {
 
 size_t mm_scan_scratch_words(uint64_t n) { return (n + kScanChunk - 1) / kScanChunk + 1; }
 
-cudaError_t launch_mm_scan(uint32_t* counts, uint32_t* offsets, uint64_t n, uint32_t* partials,
-                           cudaStream_t stream, int* launches) {
+cudaError_t launch_mm_scan(uint32_t* counts, uint64_t* ranges, uint64_t n, uint32_t* partials,
+                           bool ranked, cudaStream_t stream, int* launches) {
   int nblocks = (int)((n + kScanChunk - 1) / kScanChunk);
   if (nblocks < 1) nblocks = 1;
   mm_scan_partials<<<nblocks, kThreads, 0, stream>>>(counts, n, partials);
   mm_scan_top<<<1, kThreads, 0, stream>>>(partials, nblocks);
-  mm_scan_final<<<nblocks, kThreads, 0, stream>>>(counts, offsets, n, partials);
+  mm_scan_final<<<nblocks, kThreads, 0, stream>>>(counts, ranges, n, partials, ranked ? 1 : 0);
   *launches += 3;
   return cudaGetLastError();
 }

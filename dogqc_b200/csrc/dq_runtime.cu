@@ -37,8 +37,8 @@ int pipeline_occupancy(int smem_bytes);
 cudaError_t launch_row(const DevPipe& P, int grid, cudaStream_t stream);
 int row_occupancy(int smem_bytes);
 size_t mm_scan_scratch_words(uint64_t n);
-cudaError_t launch_mm_scan(uint32_t* counts, uint32_t* offsets, uint64_t n, uint32_t* partials,
-                           cudaStream_t stream, int* launches);
+cudaError_t launch_mm_scan(uint32_t* counts, uint64_t* ranges, uint64_t n, uint32_t* partials,
+                           bool ranked, cudaStream_t stream, int* launches);
 cudaError_t launch_heavy_prefix(const DevHeavy& H, uint64_t exp_cap, int32_t* status, cudaStream_t stream);
 cudaError_t launch_heavy_group(const DevHeavy& H, int32_t* status, int sms, cudaStream_t stream);
 size_t batch_scan_blocks(uint64_t n);
@@ -291,7 +291,9 @@ struct ResRec {
   dq_resource desc{};
   std::string name;
   DevRes dev{};
-  DevBuf slots, counts, offsets, scan_scratch;
+  DevBuf slots, counts, ranges, scan_scratch, rank;
+  bool ranked = false;      // MULTI: the count pass leaves ranks for the scatter pass
+  uint64_t src_rows = 0;    // MULTI: rows of the source its build pipelines scan
   std::vector<std::unique_ptr<DevBuf>> pay;
   uint64_t pay_rows = 0;
   int pct = 100;            // UNIQUE: slots as a percentage of the plan's capacity
@@ -603,12 +605,36 @@ void setup_resource(dq_plan* plan, ResRec& r, int64_t build_rows_bound) {
       if (cap >= 0xffffffffull) throw DqError(DQ_ERR_UNSUPPORTED, "multimaps hold fewer than 2^32 buckets");
       R.cap = cap;
       r.counts.alloc(cap * 4);
-      r.offsets.alloc((cap + 1) * 4);
+      r.ranges.alloc((cap + 1) * 8);
       R.counts = r.counts.as<uint32_t>();
-      R.offsets = r.offsets.as<uint32_t>();
+      R.ranges = r.ranges.as<uint64_t>();
       r.scan_scratch.alloc(mm_scan_scratch_words(cap) * 4);
       r.pay_rows = (uint64_t)std::max<int64_t>(build_rows_bound, 1);
+      R.pay_rows = r.pay_rows;
+      R.ranked = r.ranked ? 1 : 0;
+      if (r.ranked) {
+        r.rank.alloc(std::max<uint64_t>(r.src_rows, 1) * 4);
+        R.rank = r.rank.as<uint32_t>();
+      }
       r.pay.clear();
+      // payload rows of at most 16 bytes are one aligned item each (generated
+      // kernels): a scattered row is one store to one sector and a matched one
+      // one load, where columns would take one each per field
+      int bytes = 0;
+      for (int w : {8, 4, 2, 1})
+        for (int j = 0; j < d.npay; ++j)
+          if (R.pay_width[j] == w) {
+            R.pay_off[j] = (int8_t)std::min(bytes, 64);
+            bytes += w;
+          }
+      if (bytes > 0 && bytes <= 16 && !(plan->ctx->cfg.flags & (DQ_CFG_NO_JIT | DQ_CFG_ROW_KERNEL))) {
+        R.row_bytes = bytes <= 4 ? 4 : bytes <= 8 ? 8 : 16;
+        r.pay.emplace_back(new DevBuf());
+        r.pay.back()->alloc(r.pay_rows * (uint64_t)R.row_bytes);
+        for (int j = 0; j < d.npay; ++j)
+          R.pay[j] = r.pay.back()->ptr ? r.pay.back()->as<uint8_t>() + R.pay_off[j] : nullptr;
+        break;
+      }
       for (int j = 0; j < d.npay; ++j) {
         r.pay.emplace_back(new DevBuf());
         r.pay.back()->alloc(r.pay_rows * ctype_width(d.pay_ctype[j]));
@@ -1380,7 +1406,8 @@ int enqueue_run(dq_plan* plan, cudaStream_t st, int32_t* host_status, bool fast 
     }
     if (p.mm_count) {
       ResRec& r = *plan->res[p.mm_res];
-      DQ_CUDA(launch_mm_scan(r.dev.counts, r.dev.offsets, r.dev.cap, r.scan_scratch.as<uint32_t>(), st, &launches));
+      DQ_CUDA(launch_mm_scan(r.dev.counts, r.dev.ranges, r.dev.cap, r.scan_scratch.as<uint32_t>(), r.ranked, st,
+                             &launches));
     }
     DQ_CUDA(cudaEventRecord(plan->events[2 + 2 * i], st));
   }
@@ -1613,7 +1640,7 @@ uint64_t plan_bytes(const dq_plan* plan) {
   uint64_t b = plan->status.bytes;
   for (auto& rp : plan->res) {
     const ResRec& r = *rp;
-    b += r.slots.bytes + r.counts.bytes + r.offsets.bytes + r.scan_scratch.bytes;
+    b += r.slots.bytes + r.counts.bytes + r.ranges.bytes + r.scan_scratch.bytes + r.rank.bytes;
     for (auto& p : r.pay) b += p->bytes;
   }
   for (auto& pp : plan->pipes) {
@@ -1766,8 +1793,10 @@ std::unique_ptr<dq_plan> make_plan(dq_ctx* ctx, const dq_plan_desc* desc, const 
     plan->cursors = reinterpret_cast<uint64_t*>(plan->status.as<uint8_t>() + 8 + 8 * (size_t)desc->npipes);
     if (plan->nprofile) plan->profile = reinterpret_cast<uint64_t*>(plan->status.as<uint8_t>() + ctrl);
   }
-  // row bound for multimap payloads: rows of the source of the pipeline that scatters into it
+  // row bound for multimap payloads: rows of the source of the pipeline that scatters into it.
+  // Ranked (generated kernels): both build pipelines scan the same source, a row of it each.
   std::vector<int64_t> bound(desc->nres, 1);
+  std::vector<int> ranked(desc->nres, (ctx->cfg.flags & (DQ_CFG_NO_JIT | DQ_CFG_ROW_KERNEL)) ? 0 : 1), built(desc->nres, -1);
   for (int i = 0; i < desc->npipes; ++i) {
     const dq_pipeline& d = desc->pipes[i];
     if (d.nops <= 0 || d.nops > DQ_MAX_OPS) throw DqError(DQ_ERR_BAD_IR, "bad op count");
@@ -1779,8 +1808,19 @@ std::unique_ptr<dq_plan> make_plan(dq_ctx* ctx, const dq_plan_desc* desc, const 
         if (it != ctx->tables.end()) rows = it->second.nrows;
       } else if (d.source_kind == DQ_SRC_OUTPUT && d.source_res >= 0 && d.source_res < desc->nres) {
         rows = desc->res[d.source_res].capacity;
+      } else if (d.source_kind == DQ_SRC_AGG && d.source_res >= 0 && d.source_res < desc->nres) {
+        rows = std::max<int64_t>(rows, desc->res[d.source_res].capacity + 1);
       }
       bound[sink.res] = std::max(bound[sink.res], rows);
+      for (int k = 0; k < d.nops; ++k)
+        if (d.ops[k].kind == DQ_OP_EXPAND) ranked[sink.res] = 0;
+      if (built[sink.res] >= 0) {
+        const dq_pipeline& f = desc->pipes[built[sink.res]];
+        if (f.source_kind != d.source_kind || f.source_res != d.source_res ||
+            std::string(f.table ? f.table : "") != (d.table ? d.table : ""))
+          ranked[sink.res] = 0;
+      }
+      built[sink.res] = i;
     }
   }
   for (int i = 0; i < desc->nres; ++i) {
@@ -1791,6 +1831,8 @@ std::unique_ptr<dq_plan> make_plan(dq_ctx* ctx, const dq_plan_desc* desc, const 
     r->desc.name = nullptr;
     if (!(ctx->cfg.flags & (DQ_CFG_NO_JIT | DQ_CFG_ROW_KERNEL)) && !ctx->offline && !t_offline)
       choose_bitmap(ctx, desc, i, *r);
+    r->ranked = r->desc.kind == DQ_RES_MULTI && ranked[i] && built[i] >= 0;
+    r->src_rows = (uint64_t)bound[i];
     setup_resource(plan.get(), *r, bound[i]);
     plan->res.push_back(std::move(r));
   }
@@ -1837,6 +1879,34 @@ std::unique_ptr<dq_plan> make_plan(dq_ctx* ctx, const dq_plan_desc* desc, const 
   return plan;
 }
 
+// Multimaps whose build pipelines scan a temp or aggregation table that grew,
+// or (after an overflowing run) whose build produced more rows than its source
+// has, get room for them.
+void grow_multimaps(dq_plan* plan, bool overflowed) {
+  for (auto& pp : plan->pipes) {
+    const dq_pipeline& d = pp->desc;
+    const dq_op& sink = d.ops[d.nops - 1];
+    if (sink.kind != DQ_OP_MM_COUNT) continue;
+    ResRec& r = *plan->res[sink.res];
+    uint64_t src = r.src_rows, need = r.pay_rows;
+    if (d.source_kind == DQ_SRC_OUTPUT) src = std::max(src, plan->res[d.source_res]->dev.cap);
+    if (d.source_kind == DQ_SRC_AGG) src = std::max(src, plan->res[d.source_res]->dev.cap + 1);
+    need = std::max(need, src);
+    if (overflowed) {
+      uint32_t rows = 0;  // the buckets' total
+      DQ_CUDA(cudaMemcpy(&rows, r.dev.ranges + r.dev.cap, 4, cudaMemcpyDeviceToHost));
+      need = std::max<uint64_t>(need, rows);
+    }
+    if (src <= r.src_rows && need <= r.pay_rows) continue;
+    r.src_rows = src;
+    r.desc.capacity = (int64_t)r.dev.cap;  // the buckets stay (multi_pct is in them already)
+    const int pct = plan->opts.multi_pct;
+    plan->opts.multi_pct = 100;
+    setup_resource(plan, r, (int64_t)need);
+    plan->opts.multi_pct = pct;
+  }
+}
+
 // Grows the tables a failed run overflowed (device status bits) and re-derives
 // the pipelines' descriptors.
 void grow_plan(dq_plan* plan, int status) {
@@ -1863,6 +1933,7 @@ void grow_plan(dq_plan* plan, int status) {
       }
     }
   }
+  grow_multimaps(plan, (status & kErrOverflow) != 0);
   refresh_pipelines(plan);
 }
 
@@ -2059,8 +2130,9 @@ void build_batch(dq_batch* b, const jit::Tuning& tuning, cudaStream_t st) {
       for (int i = 0; i < b->ninst; ++i) {
         const DevRes& R = b->inst[i]->res[p0.mm_res]->dev;
         segs[i].counts = R.counts;
-        segs[i].offsets = R.offsets;
+        segs[i].ranges = R.ranges;
         segs[i].n = R.cap;
+        segs[i].ranked = R.ranked;
         segs[i].block0 = blocks;
         segs[i].nblocks = batch_scan_blocks(R.cap);
         blocks += segs[i].nblocks;
@@ -2987,7 +3059,9 @@ uint64_t estimate_bytes(dq_ctx* ctx, const dq_plan_desc& d) {
             if (it != ctx->tables.end()) rows = (uint64_t)it->second.nrows;
           }
         }
-        b += cap * 8 + rows * widths + 256;
+        // counts and ranges, ranks, payload items or columns
+        const uint64_t item = widths <= 4 ? 4 : widths <= 8 ? 8 : widths <= 16 ? 16 : widths;
+        b += cap * 12 + rows * (4 + item) + 1024;
         multi_rows[i] = rows;
         break;
       }
@@ -3427,8 +3501,9 @@ void srv_dispatch_batch(dq_server* s, SrvSlot& slot, SrvShape* sh) {
       for (int i = 0; i < K; ++i) {
         const DevRes& R = B.members[i].second->plan->res[S.mm_res]->dev;
         segs[i].counts = R.counts;
-        segs[i].offsets = R.offsets;
+        segs[i].ranges = R.ranges;
         segs[i].n = R.cap;
+        segs[i].ranked = R.ranked;
         segs[i].block0 = blocks;
         segs[i].nblocks = batch_scan_blocks(R.cap);
         blocks += segs[i].nblocks;

@@ -1,0 +1,92 @@
+"""Multimap builds whose scatter places rows by the ranks of the count pass:
+payloads of every width class, keys from unique to one hot key, row counts at
+the edges of a step, filters before the sink, aggregated and temp-table
+sources, and a build side whose rows outgrow the plan's estimate."""
+import numpy as np
+import pytest
+
+from canonical import canonical_rows
+from evaluator import run_plan
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def engine():
+    from dogqc_b200.engine import Engine
+    e = Engine(0)
+    yield e
+    e.close()
+
+
+def _db(n, distinct, hot, seed):
+    from dogqc_b200.database import Database, Table
+    from dogqc_b200.types import Type
+    r = np.random.default_rng(seed)
+    key = r.integers(1, distinct + 1, n).astype(np.int32)
+    key[r.random(n) < hot] = 1
+    build = {"k": key, "c": r.integers(-100, 100, n).astype(np.int8), "i": r.integers(-1000, 1000, n, dtype=np.int32),
+             "d": r.integers(0, 1 << 30, n).astype(np.uint32), "m": r.integers(0, 1 << 50, n).astype(np.uint64),
+             "m2": r.integers(0, 1 << 50, n).astype(np.uint64)}
+    probe = {"p": r.integers(0, distinct + 3, max(n // 4, 3), dtype=np.int32)}
+    T = Type
+    return Database([Table("b", build, {"k": T.INT, "c": T.CHAR, "i": T.INT, "d": T.DATE, "m": T.FLOAT, "m2": T.FLOAT}),
+                     Table("p", probe, {"p": T.INT})])
+
+
+def _check(engine, db, plan):
+    engine.register_database(db, force=True)
+    p = engine.prepare(plan)
+    want = canonical_rows(run_plan(db, plan)[1])
+    for _ in range(3):
+        assert canonical_rows(p.execute().rows()) == want
+    p.free()
+
+
+@pytest.mark.parametrize("n,distinct,hot", [(1, 1, 0), (1023, 2000, 0), (1025, 40, 0.5), (4096, 1, 1.0), (30_001, 9000, 0.02),
+                                            (30_000, 30_000, 0.9)])
+@pytest.mark.parametrize("fields", ["", "c", "c i", "d m", "m m2 c", "c i d m"])
+@pytest.mark.parametrize("cut", [None, 500])
+def test_payloads(engine, n, distinct, hot, fields, cut):
+    import dogqc_b200.scalar as scal
+    from dogqc_b200.relational import Reduction, RelationalAlgebra
+    from dogqc_b200.types import Type
+    db = _db(n, distinct, hot, n + distinct)
+    alg = RelationalAlgebra(db)
+    build, cfg = alg.scan("b"), {}
+    if cut is not None:
+        build = alg.selection(scal.SmallerExpr(scal.AttrExpr("i"), scal.ConstExpr(str(cut), Type.INT)), build)
+        cfg[build.opId] = {"selectivity": 0.4}
+    j = alg.join(("k", "p"), build, alg.scan("p"))
+    sums = [(Reduction.SUM, f, "s" + f) for f in fields.split()]
+    agg = alg.aggregation([], [(Reduction.COUNT, "", "n")] + sums, j)
+    _check(engine, db, alg.resolveAlgebraPlan(agg, cfg))
+
+
+@pytest.mark.parametrize("groups", [16, 1, 100_000])
+def test_build_side_from_an_aggregation(engine, groups):
+    """The build side is an aggregation's groups, staged in a temp table whose
+    estimate may be far too small."""
+    from dogqc_b200.relational import Reduction, RelationalAlgebra
+    db = _db(20_000, 6000, 0, 5)
+    alg = RelationalAlgebra(db)
+    per = alg.aggregation(["k"], [(Reduction.SUM, "m", "t"), (Reduction.COUNT, "", "c1")], alg.scan("b"))
+    j = alg.join(("k", "p"), per, alg.scan("p"))
+    agg = alg.aggregation([], [(Reduction.COUNT, "", "n"), (Reduction.SUM, "t", "tt")], j)
+    _check(engine, db, alg.resolveAlgebraPlan(agg, {per.opId: {"numgroups": groups}}))
+
+
+@pytest.mark.parametrize("selectivity", [0.9, 0.00001])
+def test_staged_build_side_outgrows_its_estimate(engine, selectivity):
+    """A costly build side (its LIKE keeps it in one pass) estimated at a few
+    rows: the temp table, the payload and the ranks grow, and the run repeats."""
+    import dogqc_b200.scalar as scal
+    from dogqc_b200 import workloads as W
+    from dogqc_b200.relational import RelationalAlgebra
+    from dogqc_b200.relational import Reduction
+    from dogqc_b200.types import Type
+    db = W.gen_tpch(0.01)
+    alg = RelationalAlgebra(db)
+    plan, cfg = W.plan_c17(alg, scal, Type, Reduction, numgroups=2000)
+    cfg = {k: dict(v, selectivity=selectivity) if "selectivity" in v else v for k, v in cfg.items()}
+    _check(engine, db, alg.resolveAlgebraPlan(plan, cfg))
