@@ -48,6 +48,11 @@ constexpr int kPrivateMax = 68 * 1024;      // shared memory per-thread accumula
 constexpr int kPrivateSlots = 64;           // group slots beside them
 constexpr int kBlock = kThreads;
 constexpr int kTailChunk = 8;               // slots a thread of a fused tail looks at together
+// Kernels whose CTAs stage bitmaps of this size take 512 threads and two CTAs an
+// SM: half as many copies, and a fixed 32 warps an SM, beside the bits that are
+// probed in place through L1 (the 60 M-row star join's fact kernel: 256 threads
+// 510 us at any occupancy, 128 threads 414, 512 threads and two CTAs 340).
+constexpr int kWideBits = 8 * 1024;
 constexpr int kWarpBuf = 64;                // rows one warp's divergence buffer holds
 constexpr int kStrSlotWords = 6;            // a CTA-local group slot's string: 4 words, length, location
 
@@ -2042,6 +2047,15 @@ struct Gen {
     bitmap_init();
   }
 
+  // Bytes of key-domain bitmaps a CTA of this pipeline's kernel holds.
+  int staged_bits() const {
+    int bytes = 0;
+    for (int k = 0; k < P.nops; ++k)
+      if (P.ops[k].kind == DQ_OP_PROBE && P.res[P.ops[k].res].bitmap == 1 && P.res[P.ops[k].res].cap <= 8192)
+        bytes += (int)P.res[P.ops[k].res].cap * 4;
+    return bytes;
+  }
+
   // The key-domain bitmaps of at most 32 KB this kernel probes, one word per
   // thread into shared memory (a probe is then a bank access, not an L2
   // access); larger ones are probed in place.
@@ -2582,6 +2596,7 @@ Program generate(const DevPipe& P, int expand_op, int refill_op, const Tuning& t
   g.patterns = patterns;
   g.batched = t.batched;
   if (t.block == 128 || t.block == 256 || t.block == 512) g.block = t.block;
+  else if (!t.batched && g.staged_bits() >= kWideBits) g.block = 512, g.min_blocks = 2;
   if (t.min_blocks > 0 && t.min_blocks * g.block <= 2048) g.min_blocks = t.min_blocks;
   bool has_expand = false;
   for (int i = 0; i < P.nops; ++i) has_expand |= P.ops[i].kind == DQ_OP_EXPAND;
