@@ -1245,6 +1245,10 @@ struct Gen {
     L(ec + " = (uint32_t)(xr_ >> 32);");
     --ind;
     L("}");
+    // a warp whose rows meet nothing goes on at once (16.8 M probes, one in a
+    // thousand with a match: 236 -> 233 us a pass)
+    L("if (__any_sync(kFull, " + ec + " != 0u)) {");
+    ++ind;
     if (k == expand_op && level == 0) {
       // deferral of long ranges: one atomic per warp reserves the item slots
       L("{");
@@ -1332,6 +1336,8 @@ struct Gen {
       row = nr;
     }
     pairs(k, level + 1, a, m, "continue;");
+    --ind;
+    L("}");
     --ind;
     L("}");
     --ind;
