@@ -123,6 +123,8 @@ struct DevRes {
                           //    (1 << 32) | payload, 0 when the key is absent
   int64_t bmin;
   uint64_t brange;
+  uint32_t* bits;         // MULTI, filter: a bit per key of [bmin, bmin + brange) that
+  int32_t filter;         // the build side holds (set by the count pass)
 };
 
 struct DevHeavy {         // deferred wide expansion ranges

@@ -201,7 +201,12 @@ struct Gen {
   int hot_off = 0;               // shared-memory offset of that table
   std::string inst_expr = "0u";  // the instance a deferred item belongs to (batches)
   std::string ldfn = "__ldcs";   // load function of streamed source columns
-  std::vector<std::pair<int, int>> bitmaps;  // key-domain bitmaps probed: (resource, smem offset)
+  struct Staged {                // key-domain bits a CTA holds in shared memory
+    int res, off;
+    long long words;
+    std::string bits;            // where they are in global memory
+  };
+  std::vector<Staged> bitmaps;
   const std::string* patterns = nullptr;     // host copy of the pattern bytes (P.pat_off into it)
   std::vector<std::string> str_ptr, str_len;  // located string keys of the last str_key_hashes
   std::vector<std::string> str_words;         // and their words (strings of at most kStrCoopMin bytes)
@@ -1196,7 +1201,7 @@ struct Gen {
     ++ind;
     std::string kk = keys(op, r, op.list, op.nlist);
     L("const uint32_t b_ = " + bucket(op, r, kk, sh) + ";");
-    L("const uint64_t xr_ = " + res(r) + ".ranges[b_];");
+    L("const uint64_t xr_ = " + may_hold(r, kk + "[0]") + " ? " + res(r) + ".ranges[b_] : 0ull;");
     L("uint32_t " + m + " = (uint32_t)xr_;");
     L("const uint32_t " + me + " = " + m + " + (uint32_t)(xr_ >> 32);");
     L("for (; " + m + " < " + me + "; ++" + m + ") {");
@@ -1240,7 +1245,7 @@ struct Gen {
     ++ind;
     std::string kk = keys(op, r, op.list, op.nlist);
     L("const uint32_t b_ = " + bucket(op, r, kk, sh) + ";");
-    L("const uint64_t xr_ = " + res(r) + ".ranges[b_];");
+    L("const uint64_t xr_ = " + may_hold(r, kk + "[0]") + " ? " + res(r) + ".ranges[b_] : 0ull;");
     L(eo + " = (uint32_t)xr_;");
     L(ec + " = (uint32_t)(xr_ >> 32);");
     --ind;
@@ -1522,6 +1527,11 @@ struct Gen {
     ++ind;
     std::string k = keys(op, r, op.list, op.nlist);
     L("b_ = " + bucket(op, r, k, sh) + ";");
+    if (!scatter && R.filter && !batched) {
+      L("const uint64_t fo_ = (uint64_t)" + k + "[0] - (uint64_t)" + res(r) + ".bmin;");
+      L("if (fo_ < " + res(r) + ".brange) atomicOr(" + res(r) + ".bits + (fo_ >> 5), 1u << (fo_ & 31u));");
+      L("else set_status(P, kErrKeyRange);  // the table's data changed since preparation");
+    }
     --ind;
     L("}");
     std::vector<std::string> vals;
@@ -2083,22 +2093,31 @@ struct Gen {
     if (batched) return;  // a batched kernel's items change instance: its probes read the bits in place
     for (int k = 0; k < P.nops; ++k) {
       const dq_op& op = P.ops[k];
-      if (op.kind != DQ_OP_PROBE || P.res[op.res].bitmap != 1 || P.res[op.res].cap > 8192) continue;
+      long long words = 0;
+      std::string bits;
+      if (op.kind == DQ_OP_PROBE && P.res[op.res].bitmap == 1) {
+        words = (long long)P.res[op.res].cap;
+        bits = "reinterpret_cast<const uint32_t*>(" + res(op.res) + ".slots)";
+      } else if ((op.kind == DQ_OP_EXPAND || op.kind == DQ_OP_EXISTS) && P.res[op.res].filter) {
+        words = ((long long)P.res[op.res].brange + 31) / 32;
+        bits = res(op.res) + ".bits";
+      }
+      if (words <= 0 || words > 8192) continue;
       bool seen = false;
-      for (auto& b : bitmaps) seen |= b.first == op.res;
+      for (auto& b : bitmaps) seen |= b.res == op.res;
       if (seen) continue;
       const int off = (smem + 15) / 16 * 16;
-      bitmaps.emplace_back(op.res, off);
-      smem = off + (int)P.res[op.res].cap * 4;
+      bitmaps.push_back({op.res, off, words, bits});
+      smem = off + (int)words * 4;
     }
   }
 
   void bitmap_init() {
     for (auto& b : bitmaps) {
       L("{");
-      L("  const uint32_t* g_ = reinterpret_cast<const uint32_t*>(" + res(b.first) + ".slots);");
-      L("  uint32_t* s_ = reinterpret_cast<uint32_t*>(smem + " + num(b.second) + ");");
-      L("  for (uint32_t i = tid; i < (uint32_t)" + res(b.first) + ".cap; i += " + num(block) + "u) s_[i] = __ldcg(g_ + i);");
+      L("  const uint32_t* g_ = " + b.bits + ";");
+      L("  uint32_t* s_ = reinterpret_cast<uint32_t*>(smem + " + num(b.off) + ");");
+      L("  for (uint32_t i = tid; i < " + num(b.words) + "u; i += " + num(block) + "u) s_[i] = __ldcg(g_ + i);");
       L("}");
     }
     if (!bitmaps.empty()) L("__syncthreads();");
@@ -2107,8 +2126,25 @@ struct Gen {
   // Bits of resource r as the probe reads them: shared memory or in place.
   std::string bitmap_words(int r) const {
     for (auto& b : bitmaps)
-      if (b.first == r) return "reinterpret_cast<const uint32_t*>(smem + " + num(b.second) + ")";
+      if (b.res == r) return "reinterpret_cast<const uint32_t*>(smem + " + num(b.off) + ")";
     return "reinterpret_cast<const uint32_t*>(" + res(r) + ".slots)";
+  }
+
+  // Whether a multimap probe asks the staged bits of the build side's keys
+  // first: a random load of a bucket's range costs the SM's L1 a cycle a lane, a
+  // bit in shared memory a few cycles a warp, and a selective build side leaves
+  // most buckets empty (16.8 M probes of 4,500 rows' keys in 100,000: 116 -> 105 us).
+  bool filtered(int r) const {
+    for (auto& b : bitmaps)
+      if (b.res == r && P.res[r].filter) return true;
+    return false;
+  }
+
+  // The test that key value `key` may be in multimap r ("true" without bits).
+  std::string may_hold(int r, const std::string& key) const {
+    if (!filtered(r)) return "true";
+    const std::string o = "((uint64_t)" + key + " - (uint64_t)" + res(r) + ".bmin)";
+    return "(" + o + " < " + res(r) + ".brange && ((" + bitmap_words(r) + "[" + o + " >> 5] >> (" + o + " & 31u)) & 1u))";
   }
 
   // A word of the aggregation table the pipeline scans.  The fused tail reads

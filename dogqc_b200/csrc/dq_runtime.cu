@@ -292,6 +292,9 @@ struct ResRec {
   std::string name;
   DevRes dev{};
   DevBuf slots, counts, ranges, scan_scratch, rank;
+  DevBuf bits;
+  bool filter = false;      // MULTI: a bit per key of the build column's domain
+                            //   [bmin, bmin + brange) tells probes which keys it holds
   bool ranked = false;      // MULTI: the count pass leaves ranks for the scatter pass
   uint64_t src_rows = 0;    // MULTI: rows of the source its build pipelines scan
   std::vector<std::unique_ptr<DevBuf>> pay;
@@ -612,6 +615,13 @@ void setup_resource(dq_plan* plan, ResRec& r, int64_t build_rows_bound) {
       r.pay_rows = (uint64_t)std::max<int64_t>(build_rows_bound, 1);
       R.pay_rows = r.pay_rows;
       R.ranked = r.ranked ? 1 : 0;
+      if (r.filter && !r.no_bitmap) {
+        R.filter = 1;
+        R.bmin = r.bmin;
+        R.brange = r.brange;
+        r.bits.alloc((r.brange + 31) / 32 * 4);
+        R.bits = r.bits.as<uint32_t>();
+      }
       if (r.ranked) {
         r.rank.alloc(std::max<uint64_t>(r.src_rows, 1) * 4);
         R.rank = r.rank.as<uint32_t>();
@@ -1221,6 +1231,7 @@ void add_resets(std::vector<BatchReset>& ops, const ResRec& r) {
     }
     case DQ_RES_MULTI:
       add_fill(ops, R.counts, r.counts.bytes, 0);
+      if (R.filter) add_fill(ops, R.bits, r.bits.bytes, 0);
       break;
     default:
       break;
@@ -1640,7 +1651,8 @@ uint64_t plan_bytes(const dq_plan* plan) {
   uint64_t b = plan->status.bytes;
   for (auto& rp : plan->res) {
     const ResRec& r = *rp;
-    b += r.slots.bytes + r.counts.bytes + r.ranges.bytes + r.scan_scratch.bytes + r.rank.bytes;
+    b += r.slots.bytes + r.counts.bytes + r.ranges.bytes + r.scan_scratch.bytes + r.rank.bytes +
+         r.bits.bytes;
     for (auto& p : r.pay) b += p->bytes;
   }
   for (auto& pp : plan->pipes) {
@@ -1702,6 +1714,19 @@ bool fusable_tail(const dq_plan_desc* desc, const std::vector<std::unique_ptr<Re
   return true;
 }
 
+// The smallest and largest value of an integer column (false: no rows).
+bool column_range(dq_ctx* ctx, const ColRec& c, uint64_t rows, long long* got) {
+  DevBuf mm;
+  mm.alloc(16);
+  const long long init[2] = {LLONG_MAX, LLONG_MIN};
+  DQ_CUDA(cudaMemcpy(mm.ptr, init, 16, cudaMemcpyHostToDevice));
+  DQ_CUDA(launch_col_minmax(c.data->as<uint8_t>(), rows, ctype_width(c.ctype), c.ctype != DQ_U32, mm.as<long long>(),
+                            ctx->sms, ctx->stream));
+  DQ_CUDA(cudaMemcpyAsync(got, mm.ptr, 16, cudaMemcpyDeviceToHost, ctx->stream));
+  DQ_CUDA(cudaStreamSynchronize(ctx->stream));
+  return got[0] <= got[1];
+}
+
 // Unique tables over a small key domain need no hashing: one key, read
 // straight from a column of a registered table by the one pipeline that builds
 // the table, whose smallest and largest values (measured on the device at
@@ -1751,21 +1776,50 @@ void choose_bitmap(dq_ctx* ctx, const dq_plan_desc* desc, int i, ResRec& r) {
   const ColRec* c = t->second.find(build->cols[ci]);
   // the key is the column's value unchanged: same type in the slot and the table
   if (!c || c->ctype != kt || build->slots[ks].ctype != kt || !c->data || !c->data->ptr) return;
-  DevBuf mm;
-  mm.alloc(16);
-  const long long init[2] = {LLONG_MAX, LLONG_MIN};
-  DQ_CUDA(cudaMemcpy(mm.ptr, init, 16, cudaMemcpyHostToDevice));
-  DQ_CUDA(launch_col_minmax(c->data->as<uint8_t>(), (uint64_t)t->second.nrows, ctype_width(c->ctype),
-                            kt != DQ_U32, mm.as<long long>(), ctx->sms, ctx->stream));
   long long got[2];
-  DQ_CUDA(cudaMemcpyAsync(got, mm.ptr, 16, cudaMemcpyDeviceToHost, ctx->stream));
-  DQ_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (got[0] > got[1]) return;
+  if (!column_range(ctx, *c, (uint64_t)t->second.nrows, got)) return;
   const uint64_t span = (uint64_t)got[1] - (uint64_t)got[0] + 1;  // 0: all 2^64 values
   const uint64_t rows = (uint64_t)t->second.nrows;
   if (span == 0 || span > kDenseKeys || (d.npay == 0 ? span > kBitmapKeys && span > 64 * rows : span > 4 * rows))
     return;
   r.bitmap = d.npay == 0 ? 1 : 2;
+  r.bmin = got[0];
+  r.brange = span;
+}
+
+// Multimaps probed through bits of their keys: one key of at most 32 bits,
+// read straight from a column of a registered table whose values (measured at
+// preparation) span at most kBitmapKeys keys, so that the bits fit a CTA's
+// shared memory, and a build side that keeps few of the table's rows (the plan
+// asks for fewer buckets than a quarter of them): the bits are set by an atomic
+// a kept row, which many rows of few keys would queue up at.
+void choose_filter(dq_ctx* ctx, const dq_plan_desc* desc, int i, ResRec& r) {
+  const dq_resource& d = desc->res[i];
+  if (d.kind != DQ_RES_MULTI || d.nkeys != 1) return;
+  const int kt = d.key_ctype[0];
+  if (kt != DQ_I8 && kt != DQ_I32 && kt != DQ_U32) return;
+  const dq_pipeline* build = nullptr;
+  for (int p = 0; p < desc->npipes; ++p) {
+    const dq_op& sink = desc->pipes[p].ops[desc->pipes[p].nops - 1];
+    if (sink.kind == DQ_OP_MM_COUNT && sink.res == i) build = &desc->pipes[p];
+  }
+  if (!build || build->source_kind != DQ_SRC_TABLE || !build->table) return;
+  const dq_op& sink = build->ops[build->nops - 1];
+  if (sink.nlist != 1 || sink.list < 0 || sink.list >= build->nlist) return;
+  const int ks = build->lists[sink.list];
+  if (ks < 0 || ks >= build->nslots || build->slots[ks].kind != DQ_SLOT_COL) return;
+  const int ci = build->slots[ks].src;
+  if (ci < 0 || ci >= build->ncols || !build->cols[ci]) return;
+  auto t = ctx->tables.find(build->table);
+  if (t == ctx->tables.end() || t->second.nrows <= 0) return;
+  const ColRec* c = t->second.find(build->cols[ci]);
+  if (!c || c->ctype != kt || build->slots[ks].ctype != kt || !c->data || !c->data->ptr) return;
+  if (d.capacity * 4 > t->second.nrows) return;
+  long long got[2];
+  if (!column_range(ctx, *c, (uint64_t)t->second.nrows, got)) return;
+  const uint64_t span = (uint64_t)got[1] - (uint64_t)got[0] + 1;
+  if (span > kBitmapKeys) return;
+  r.filter = true;
   r.bmin = got[0];
   r.brange = span;
 }
@@ -1833,6 +1887,7 @@ std::unique_ptr<dq_plan> make_plan(dq_ctx* ctx, const dq_plan_desc* desc, const 
       choose_bitmap(ctx, desc, i, *r);
     r->ranked = r->desc.kind == DQ_RES_MULTI && ranked[i] && built[i] >= 0;
     r->src_rows = (uint64_t)bound[i];
+    if (r->ranked && !ctx->offline && !t_offline && !opts.batch_member) choose_filter(ctx, desc, i, *r);
     setup_resource(plan.get(), *r, bound[i]);
     plan->res.push_back(std::move(r));
   }
@@ -1879,6 +1934,15 @@ std::unique_ptr<dq_plan> make_plan(dq_ctx* ctx, const dq_plan_desc* desc, const 
   return plan;
 }
 
+// Lays a multimap out again for `rows` payload rows; its buckets stay.
+void resize_multimap(dq_plan* plan, ResRec& r, uint64_t rows) {
+  r.desc.capacity = (int64_t)r.dev.cap;  // multi_pct is in it already
+  const int pct = plan->opts.multi_pct;
+  plan->opts.multi_pct = 100;
+  setup_resource(plan, r, (int64_t)rows);
+  plan->opts.multi_pct = pct;
+}
+
 // Multimaps whose build pipelines scan a temp or aggregation table that grew,
 // or (after an overflowing run) whose build produced more rows than its source
 // has, get room for them.
@@ -1899,11 +1963,7 @@ void grow_multimaps(dq_plan* plan, bool overflowed) {
     }
     if (src <= r.src_rows && need <= r.pay_rows) continue;
     r.src_rows = src;
-    r.desc.capacity = (int64_t)r.dev.cap;  // the buckets stay (multi_pct is in them already)
-    const int pct = plan->opts.multi_pct;
-    plan->opts.multi_pct = 100;
-    setup_resource(plan, r, (int64_t)need);
-    plan->opts.multi_pct = pct;
+    resize_multimap(plan, r, need);
   }
 }
 
@@ -1912,6 +1972,11 @@ void grow_multimaps(dq_plan* plan, bool overflowed) {
 void grow_plan(dq_plan* plan, int status) {
   for (auto& rp : plan->res) {
     ResRec& r = *rp;
+    if ((status & kErrKeyRange) && r.filter && !r.no_bitmap) {
+      r.no_bitmap = true;
+      resize_multimap(plan, r, r.pay_rows);
+      continue;
+    }
     if ((status & kErrKeyRange) && r.bitmap && !r.no_bitmap) {
       // the table's data changed since preparation: a hash table from now on
       r.no_bitmap = true;
