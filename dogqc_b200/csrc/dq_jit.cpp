@@ -53,6 +53,7 @@ constexpr int kTailChunk = 8;               // slots a thread of a fused tail lo
 // probed in place through L1 (the 60 M-row star join's fact kernel: 256 threads
 // 510 us at any occupancy, 128 threads 414, 512 threads and two CTAs 340).
 constexpr int kWideBits = 8 * 1024;
+constexpr int kRepeats = 4;                 // rows per key from which a CTA builds a bitmap's bits itself
 constexpr int kWarpBuf = 64;                // rows one warp's divergence buffer holds
 constexpr int kStrSlotWords = 6;            // a CTA-local group slot's string: 4 words, length, location
 
@@ -195,6 +196,7 @@ struct Gen {
   int refill_threshold = 32;     // buffered rows that make the warp process them
   int nbuf = 0;                  // values per row in the warp buffers
   int buf_off = 0;               // shared-memory offset of the warp buffers
+  int bits_off = -1;             // smem offset of the CTA's own bits of the bitmap it builds (-1: none)
   bool hot = false;              // ranked multimap count through the CTA's hot-bucket table
   bool steps = false;            // ranked multimap pass that handles a thread's rows of a step together
   std::map<int, std::string> item;  // multimap -> the gathered payload item of the current match
@@ -1475,8 +1477,8 @@ struct Gen {
         L("  if (o_ < " + res(r) + ".brange) reinterpret_cast<unsigned long long*>(" + res(r) +
           ".slots)[o_] = (1ull << 32) | " + pay + ";");
       } else {
-        L("  if (o_ < " + res(r) + ".brange) atomicOr(reinterpret_cast<unsigned int*>(" + res(r) +
-          ".slots) + (o_ >> 5), 1u << (o_ & 31u));");
+        const std::string w = bits_off >= 0 ? "smem + " + num(bits_off) : res(r) + ".slots";
+        L("  if (o_ < " + res(r) + ".brange) atomicOr(reinterpret_cast<unsigned int*>(" + w + ") + (o_ >> 5), 1u << (o_ & 31u));");
       }
       L("  else set_status(P, kErrKeyRange);");
       L("}");
@@ -1742,6 +1744,39 @@ struct Gen {
     if (!hot) return;
     hot_off = (smem + 15) / 16 * 16;
     smem = hot_off + kHotSlots * 12;
+  }
+
+  // A build side that repeats its keys sets the same bits of a small bitmap over
+  // and over, and atomics on one line queue up at L2: the CTA sets bits of its
+  // own in shared memory and merges them once, a line at a time.  (1.5 M rows of
+  // 100,000 keys: 40 -> 16 us.)  For build sides of at least kRepeats rows per key of
+  // the domain; with fewer, the merges of all CTAs are as many atomics.
+  void choose_own_bits() {
+    bits_off = -1;
+    if (batched || P.nops == 0 || P.source_kind != DQ_SRC_TABLE) return;
+    const dq_op& sink = P.ops[P.nops - 1];
+    if (sink.kind != DQ_OP_BUILD) return;
+    const DevRes& R = P.res[sink.res];
+    if (R.bitmap != 1 || R.cap > 8192 || P.nrows < kRepeats * (int64_t)R.brange) return;
+    bits_off = (smem + 15) / 16 * 16;
+    smem = bits_off + (int)R.cap * 4;
+  }
+
+  void own_bits_init() {
+    if (bits_off < 0) return;
+    const std::string W = num((long long)P.res[P.ops[P.nops - 1].res].cap);
+    L("for (int i = tid; i < " + W + "; i += " + num(block) + ") reinterpret_cast<uint32_t*>(smem + " + num(bits_off) + ")[i] = 0u;");
+    L("__syncthreads();");
+  }
+
+  void own_bits_flush() {
+    if (bits_off < 0) return;
+    const int r = P.ops[P.nops - 1].res;
+    L("__syncthreads();");
+    L("for (int i = tid; i < " + num((long long)P.res[r].cap) + "; i += " + num(block) + ") {");
+    L("  const uint32_t b_ = reinterpret_cast<const uint32_t*>(smem + " + num(bits_off) + ")[i];");
+    L("  if (b_) atomicOr(reinterpret_cast<unsigned int*>(" + res(r) + ".slots) + i, b_);");
+    L("}");
   }
 
   void hot_init() {
@@ -2294,6 +2329,7 @@ struct Gen {
   void main_kernel() {
     prologue("dq_main");
     hot_init();
+    own_bits_init();
     std::vector<int> cols = source_cols();
     L("const int64_t nrows = source_rows(P);");
     L("const int64_t span = " + num((long long)block * U) + ";");
@@ -2337,6 +2373,7 @@ struct Gen {
     }
     --ind;
     L("}");
+    own_bits_flush();
     epilogue();
   }
 
@@ -2673,6 +2710,7 @@ Program generate(const DevPipe& P, int expand_op, int refill_op, const Tuning& t
   g.choose_agg();
   g.choose_refill(refill_op);
   g.choose_hot();
+  g.choose_own_bits();
   g.choose_prefetch();
   g.choose_bitmaps();
   if (g.U == 4 && rows <= 0) {
@@ -2713,6 +2751,7 @@ Program generate(const DevPipe& P, int expand_op, int refill_op, const Tuning& t
     prog.batched = true;
     return prog;
   }
+  if (g.bits_off >= 0) prog.max_ctas = 2;  // a merge per CTA
   g.main_kernel();
   if (expand_op >= 0) {
     g.o += "\n";

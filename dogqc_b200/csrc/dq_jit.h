@@ -30,6 +30,7 @@ struct Program {
   int block = kThreads;      // threads per CTA
   bool heavy = false;        // second kernel for deferred expansion ranges
   bool batched = false;      // one kernel `dq_batch_main` over many instances
+  int max_ctas = 0;          // CTAs per SM worth launching (0: as many as fit)
 };
 
 struct Kernels {

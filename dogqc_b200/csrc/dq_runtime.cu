@@ -1109,6 +1109,7 @@ void setup_pipeline(dq_plan* plan, PipeRec& p) {
   if (occ < 1) throw DqError(DQ_ERR_UNSUPPORTED, "pipeline kernel cannot be resident with this shared memory");
   const int asked = plan->opts.ctas_per_sm > 0 ? plan->opts.ctas_per_sm : ctx->cfg.ctas_per_sm;
   int want = asked > 0 ? std::min(asked, occ) : occ;
+  if (p.jit && asked <= 0 && p.prog.max_ctas > 0) want = std::min(want, p.prog.max_ctas);
   p.grid_full = ctx->sms * want;
   p.grid = p.grid_full;
   if (!P.nrows_dev) {  // no more CTAs than row blocks
