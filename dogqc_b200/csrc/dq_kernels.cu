@@ -1279,7 +1279,7 @@ __global__ void mm_scan_final(uint32_t* counts, uint64_t* ranges, uint64_t n, co
   for (int k = 0; k < kScanItems; ++k) sum += v[k];
   uint32_t excl;
   block_exclusive_scan(sum, excl);
-  uint32_t run = partials[blockIdx.x] + excl;
+  uint32_t run = (partials ? partials[blockIdx.x] : 0u) + excl;
   if (whole) {
 #pragma unroll
     for (int k = 0; k < kScanItems; k += 4) {
@@ -1666,7 +1666,11 @@ size_t mm_scan_scratch_words(uint64_t n) { return (n + kScanChunk - 1) / kScanCh
 cudaError_t launch_mm_scan(uint32_t* counts, uint64_t* ranges, uint64_t n, uint32_t* partials,
                            bool ranked, cudaStream_t stream, int* launches) {
   int nblocks = (int)((n + kScanChunk - 1) / kScanChunk);
-  if (nblocks < 1) nblocks = 1;
+  if (nblocks <= 1) {  // one chunk (a nested-loop join's single bucket, small build sides)
+    mm_scan_final<<<1, kThreads, 0, stream>>>(counts, ranges, n, nullptr, ranked ? 1 : 0);
+    *launches += 1;
+    return cudaGetLastError();
+  }
   mm_scan_partials<<<nblocks, kThreads, 0, stream>>>(counts, n, partials);
   mm_scan_top<<<1, kThreads, 0, stream>>>(partials, nblocks);
   mm_scan_final<<<nblocks, kThreads, 0, stream>>>(counts, ranges, n, partials, ranked ? 1 : 0);
