@@ -1750,10 +1750,14 @@ struct Gen {
   // and over, and atomics on one line queue up at L2: the CTA sets bits of its
   // own in shared memory and merges them once, a line at a time.  (1.5 M rows of
   // 100,000 keys: 40 -> 16 us.)  For build sides of at least kRepeats rows per key of
-  // the domain; with fewer, the merges of all CTAs are as many atomics.
+  // the domain; with fewer, the merges of all CTAs are as many atomics.  Not behind
+  // an expansion: its deferred ranges reach the sink in a kernel of their own, and
+  // the table's rows say little about the pairs.
   void choose_own_bits() {
     bits_off = -1;
     if (batched || P.nops == 0 || P.source_kind != DQ_SRC_TABLE) return;
+    for (int j = 0; j < P.nops; ++j)
+      if (P.ops[j].kind == DQ_OP_EXPAND) return;
     const dq_op& sink = P.ops[P.nops - 1];
     if (sink.kind != DQ_OP_BUILD) return;
     const DevRes& R = P.res[sink.res];
