@@ -24,8 +24,14 @@ enum : int32_t {
                          // turns the table back into a hash table and re-runs
   kInfoHeavyFull = 32,   // informational: deferred expansion items exceeded their
                          // capacity; the rest ran in place (results stay exact)
+  kErrMultiFull = 64,    // a multimap's build side has more rows than there is
+                         // payload room for: nothing is scattered or probed, the
+                         // host grows the multimap and re-runs
 };
 constexpr int32_t kInfoMask = kInfoHeavyFull;
+// A run that has one of these is repeated or fails, and its tables are not
+// whole: the kernels that follow do nothing.
+constexpr int32_t kErrStop = kErrHtFull | kErrTimeout | kErrMultiFull;
 
 struct DevCol {           // staged fixed-width column
   const uint8_t* ptr;
@@ -105,7 +111,6 @@ struct DevRes {
   int32_t ranked;
   int32_t row_bytes;      // MULTI: > 0: a row's payload is one aligned item of that
                           // size (field j at pay_off[j]), else a column per field
-  uint64_t pay_rows;      // MULTI: payload rows there is room for
   int8_t pay_off[DQ_MAX_PAY];
   int32_t npay;
   int32_t naggs;
@@ -269,6 +274,8 @@ struct BatchScanSeg {     // one multimap's bucket counts -> offsets
   uint32_t* counts;
   uint64_t* ranges;
   uint64_t n;             // buckets
+  uint64_t pay_rows;      // payload rows there is room for
+  int32_t* status;
   uint64_t block0;        // first scan block of this segment
   uint64_t nblocks;
   int32_t ranked;         // the counts stay (a ranked multimap's scatter needs none)

@@ -1102,10 +1102,6 @@ struct Gen {
   void store_payload(int r, const std::string& pos, const std::vector<std::string>& v) {
     const DevRes& R = P.res[r];
     if (v.empty()) return;
-    L("if (" + pos + " >= " + res(r) + ".pay_rows) {  // more rows than were there at preparation");
-    L("  set_status(P, kErrOverflow);");
-    L("} else {");
-    ++ind;
     if (R.row_bytes > 0) {
       std::vector<std::string> word((size_t)R.row_bytes / 4);
       auto put = [&](int k, const std::string& x) { word[(size_t)k] += (word[(size_t)k].empty() ? "" : " | ") + x; };
@@ -1131,8 +1127,6 @@ struct Gen {
         L("st(" + res(r) + ".pay[" + num((long long)j) + "] + (size_t)" + pos + " * " + num(w) + ", " + num(w) + ", " + v[j] + ");");
       }
     }
-    --ind;
-    L("}");
   }
 
   // Gathers the pending payload values the given slots need (lanes that a
@@ -2107,7 +2101,7 @@ struct Gen {
       (min_blocks > 0 ? ", " + num(min_blocks) : std::string()) + ") " + name + "(const __grid_constant__ DevPipe P) {");
     ++ind;
     L("extern __shared__ __align__(16) uint8_t smem[];");
-    L("if (*(volatile int32_t*)P.status & (kErrHtFull | kErrTimeout)) return;");
+    L("if (*(volatile int32_t*)P.status & kErrStop) return;");
     L("const int tid = threadIdx.x, lane = tid & 31;");
     L("(void)smem;");
     L("(void)lane;");
@@ -2228,7 +2222,7 @@ struct Gen {
     L("__device__ __noinline__ void dq_tail(const DevPipe& P, uint16_t* list) {");
     ++ind;
     L("__shared__ uint32_t tn_, to_;  // listed slots, emitted rows");
-    L("if (*(volatile int32_t*)P.status & (kErrHtFull | kErrTimeout)) return;");
+    L("if (*(volatile int32_t*)P.status & kErrStop) return;");
     L("const int tid = threadIdx.x, lane = tid & 31;");
     L("(void)lane;");
     L("const int64_t nrows = " + (R.nkeys > 0 ? "(int64_t)" + res(sr) + ".cap + 1" : std::string("1")) + ";");
@@ -2477,7 +2471,7 @@ struct Gen {
       ") dq_batch_main(const DevPipe* __restrict__ Ps, const int64_t* __restrict__ bprefix, int ninst) {");
     ++ind;
     L("extern __shared__ __align__(16) uint8_t smem[];");
-    L("if (*(volatile int32_t*)Ps[0].status & (kErrHtFull | kErrTimeout)) return;");
+    L("if (*(volatile int32_t*)Ps[0].status & kErrStop) return;");
     L("const int tid = threadIdx.x, lane = tid & 31;");
     L("(void)smem;");
     L("(void)lane;");
@@ -2540,7 +2534,7 @@ struct Gen {
         ") dq_batch_heavy(const DevPipe* __restrict__ Ps, int ninst) {");
       ++ind;
       L("extern __shared__ __align__(16) uint8_t smem[];");
-      L("if (*(volatile int32_t*)Ps[0].status & (kErrHtFull | kErrTimeout)) return;");
+      L("if (*(volatile int32_t*)Ps[0].status & kErrStop) return;");
       L("const int tid = threadIdx.x, lane = tid & 31;");
       L("(void)smem;");
       L("(void)tid;");

@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(kThreads, 2) pipeline_kernel(const __grid_cons
   __shared__ int64_t s_tile[kMaxStages];
   // an earlier pipeline of this run overflowed a table: the host re-runs the
   // plan with larger tables, so skip the work (probing a full table is slow)
-  if (*(volatile int32_t*)P.status & (kErrHtFull | kErrTimeout)) return;
+  if (*(volatile int32_t*)P.status & kErrStop) return;
   Cta c;
   init_cta(P, c, smem);
   const int tid = threadIdx.x;
@@ -1116,7 +1116,7 @@ __device__ void row_ops(Row& x, bool act, uint8_t* smem) {
 __global__ void __launch_bounds__(kThreads, 3) row_kernel(const __grid_constant__ DevPipe Pk) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t s_mbar[kMaxStages];
-  if (*(volatile int32_t*)Pk.status & (kErrHtFull | kErrTimeout)) return;
+  if (*(volatile int32_t*)Pk.status & kErrStop) return;
   // the descriptor is indexed with runtime values in every operator: keep it in
   // shared memory rather than reading the parameter space through pointers
   {
@@ -1252,16 +1252,22 @@ __global__ void mm_scan_top(uint32_t* partials, int nblocks) {
   }
 }
 
+// Ends the run when a multimap's rows, up to `end` here, outnumber its room.
+__device__ __forceinline__ void multi_room(uint64_t end, uint64_t pay_rows, int32_t* status) {
+  if (end > pay_rows && !(*(volatile int32_t*)status & kErrMultiFull)) atomicOr(status, kErrMultiFull);
+}
+
 // Ranges of one chunk of buckets (kScanItems consecutive counts a thread, in
 // 16-byte vectors when the chunk is whole), the total behind the last one, and
 // the counts reset to zero for a scatter pass that counts again (not a ranked
-// multimap's).
-__global__ void mm_scan_final(uint32_t* counts, uint64_t* ranges, uint64_t n, const uint32_t* partials, int ranked) {
+// multimap's).  Rows past the payload's room (or past 32-bit positions: the sums
+// wrap, which the thread whose buckets cross 2^32 sees) end the run here.
+__global__ void mm_scan_final(uint32_t* counts, uint64_t* ranges, uint64_t n, const uint32_t* partials, int ranked,
+                              uint64_t pay_rows, int32_t* status) {
   static_assert(kScanItems % 4 == 0, "vector path");
   const uint64_t i0 = (uint64_t)blockIdx.x * kScanChunk + (uint64_t)threadIdx.x * kScanItems;
   const bool whole = i0 + kScanItems <= n;
   uint32_t v[kScanItems];
-  uint32_t sum = 0;
   if (whole) {
 #pragma unroll
     for (int k = 0; k < kScanItems; k += 4) {
@@ -1275,11 +1281,13 @@ __global__ void mm_scan_final(uint32_t* counts, uint64_t* ranges, uint64_t n, co
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) v[k] = (i0 + k < n) ? counts[i0 + k] : 0;
   }
+  uint64_t rows = 0;
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) sum += v[k];
+  for (int k = 0; k < kScanItems; ++k) rows += v[k];
   uint32_t excl;
-  block_exclusive_scan(sum, excl);
+  block_exclusive_scan((uint32_t)rows, excl);
   uint32_t run = (partials ? partials[blockIdx.x] : 0u) + excl;
+  multi_room(run + rows, pay_rows, status);
   if (whole) {
 #pragma unroll
     for (int k = 0; k < kScanItems; k += 4) {
@@ -1595,14 +1603,15 @@ __global__ void batch_scan_final(const BatchScanSeg* segs, int nseg, const uint3
   const BatchScanSeg s = segs[batch_seg_of(segs, nseg, b)];
   const uint64_t i0 = (b - s.block0) * kScanChunk + (uint64_t)threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
-  uint32_t sum = 0;
+  uint64_t rows = 0;
   for (int k = 0; k < kScanItems; ++k) {
     v[k] = (i0 + k < s.n) ? s.counts[i0 + k] : 0;
-    sum += v[k];
+    rows += v[k];
   }
   uint32_t excl;
-  block_exclusive_scan(sum, excl);
+  block_exclusive_scan((uint32_t)rows, excl);
   uint32_t run = partials[b] + excl;
+  multi_room(run + rows, s.pay_rows, s.status);
   for (int k = 0; k < kScanItems; ++k) {
     if (i0 + k < s.n) {
       s.ranges[i0 + k] = (uint64_t)v[k] << 32 | run;
@@ -1664,16 +1673,16 @@ int pipeline_occupancy(int smem_bytes) {
 size_t mm_scan_scratch_words(uint64_t n) { return (n + kScanChunk - 1) / kScanChunk + 1; }
 
 cudaError_t launch_mm_scan(uint32_t* counts, uint64_t* ranges, uint64_t n, uint32_t* partials,
-                           bool ranked, cudaStream_t stream, int* launches) {
+                           bool ranked, uint64_t pay_rows, int32_t* status, cudaStream_t stream, int* launches) {
   int nblocks = (int)((n + kScanChunk - 1) / kScanChunk);
   if (nblocks <= 1) {  // one chunk (a nested-loop join's single bucket, small build sides)
-    mm_scan_final<<<1, kThreads, 0, stream>>>(counts, ranges, n, nullptr, ranked ? 1 : 0);
+    mm_scan_final<<<1, kThreads, 0, stream>>>(counts, ranges, n, nullptr, ranked ? 1 : 0, pay_rows, status);
     *launches += 1;
     return cudaGetLastError();
   }
   mm_scan_partials<<<nblocks, kThreads, 0, stream>>>(counts, n, partials);
   mm_scan_top<<<1, kThreads, 0, stream>>>(partials, nblocks);
-  mm_scan_final<<<nblocks, kThreads, 0, stream>>>(counts, ranges, n, partials, ranked ? 1 : 0);
+  mm_scan_final<<<nblocks, kThreads, 0, stream>>>(counts, ranges, n, partials, ranked ? 1 : 0, pay_rows, status);
   *launches += 3;
   return cudaGetLastError();
 }

@@ -38,7 +38,7 @@ cudaError_t launch_row(const DevPipe& P, int grid, cudaStream_t stream);
 int row_occupancy(int smem_bytes);
 size_t mm_scan_scratch_words(uint64_t n);
 cudaError_t launch_mm_scan(uint32_t* counts, uint64_t* ranges, uint64_t n, uint32_t* partials,
-                           bool ranked, cudaStream_t stream, int* launches);
+                           bool ranked, uint64_t pay_rows, int32_t* status, cudaStream_t stream, int* launches);
 cudaError_t launch_heavy_prefix(const DevHeavy& H, uint64_t exp_cap, int32_t* status, cudaStream_t stream);
 cudaError_t launch_heavy_group(const DevHeavy& H, int32_t* status, int sms, cudaStream_t stream);
 size_t batch_scan_blocks(uint64_t n);
@@ -617,7 +617,6 @@ void setup_resource(dq_plan* plan, ResRec& r, int64_t build_rows_bound) {
       R.ranges = r.ranges.as<uint64_t>();
       r.scan_scratch.alloc(mm_scan_scratch_words(cap) * 4);
       r.pay_rows = (uint64_t)std::max<int64_t>(build_rows_bound, 1);
-      R.pay_rows = r.pay_rows;
       R.ranked = r.ranked ? 1 : 0;
       if (r.filter && !r.no_bitmap) {
         R.filter = 1;
@@ -1207,6 +1206,11 @@ std::vector<std::vector<int>> pipe_deps(const dq_plan* plan) {
 // replays the same launches whatever the previous replay left.
 constexpr int kLanes = 4;  // streams a captured run spreads its pipelines over
 
+// Rows a multimap's build may place: its payload's room, in 32-bit positions.
+uint64_t multi_room(const ResRec& r) {
+  return r.desc.npay == 0 ? 0xffffffffull : std::min<uint64_t>(r.pay_rows, 0xffffffffull);
+}
+
 // Appends a buffer of `bytes` to fill with 64-bit words (rounded up: device
 // buffers have padding behind them).
 void add_fill(std::vector<BatchReset>& ops, void* ptr, uint64_t bytes, uint64_t value) {
@@ -1425,8 +1429,8 @@ int enqueue_run(dq_plan* plan, cudaStream_t st, int32_t* host_status, bool fast 
     }
     if (p.mm_count) {
       ResRec& r = *plan->res[p.mm_res];
-      DQ_CUDA(launch_mm_scan(r.dev.counts, r.dev.ranges, r.dev.cap, r.scan_scratch.as<uint32_t>(), r.ranked, st,
-                             &launches));
+      DQ_CUDA(launch_mm_scan(r.dev.counts, r.dev.ranges, r.dev.cap, r.scan_scratch.as<uint32_t>(), r.ranked,
+                             multi_room(r), plan->status.as<int32_t>(), st, &launches));
     }
     DQ_CUDA(cudaEventRecord(plan->events[2 + 2 * i], st));
   }
@@ -1871,7 +1875,7 @@ std::unique_ptr<dq_plan> make_plan(dq_ctx* ctx, const dq_plan_desc* desc, const 
       } else if (d.source_kind == DQ_SRC_OUTPUT && d.source_res >= 0 && d.source_res < desc->nres) {
         rows = desc->res[d.source_res].capacity;
       } else if (d.source_kind == DQ_SRC_AGG && d.source_res >= 0 && d.source_res < desc->nres) {
-        rows = std::max<int64_t>(rows, desc->res[d.source_res].capacity + 1);
+        rows = std::max<int64_t>(desc->res[d.source_res].capacity, 16) + 1;  // its slots (setup_resource)
       }
       bound[sink.res] = std::max(bound[sink.res], rows);
       for (int k = 0; k < d.nops; ++k)
@@ -1952,8 +1956,8 @@ void resize_multimap(dq_plan* plan, ResRec& r, uint64_t rows) {
 }
 
 // Multimaps whose build pipelines scan a temp or aggregation table that grew,
-// or (after an overflowing run) whose build produced more rows than its source
-// has, get room for them.
+// or (after a run that ended for want of room) whose build produced more rows
+// than there was room for, get room for them.
 void grow_multimaps(dq_plan* plan, bool overflowed) {
   for (auto& pp : plan->pipes) {
     const dq_pipeline& d = pp->desc;
@@ -2006,7 +2010,7 @@ void grow_plan(dq_plan* plan, int status) {
       }
     }
   }
-  grow_multimaps(plan, (status & kErrOverflow) != 0);
+  grow_multimaps(plan, (status & kErrMultiFull) != 0);
   refresh_pipelines(plan);
 }
 
@@ -2068,7 +2072,7 @@ void adapt_threshold(dq_plan* plan) {
 void throw_status(int status) {
   throw DqError(status & kErrTimeout ? DQ_ERR_TIMEOUT
                 : status & kErrHtFull ? DQ_ERR_HT_FULL
-                : status & kErrOverflow ? DQ_ERR_OVERFLOW : DQ_ERR_BAD_IR,
+                : status & (kErrOverflow | kErrMultiFull) ? DQ_ERR_OVERFLOW : DQ_ERR_BAD_IR,
                 "device status " + std::to_string(status));
 }
 
@@ -2217,6 +2221,8 @@ void build_batch(dq_batch* b, const jit::Tuning& tuning, cudaStream_t st) {
         segs[i].counts = R.counts;
         segs[i].ranges = R.ranges;
         segs[i].n = R.cap;
+        segs[i].pay_rows = multi_room(*b->inst[i]->res[p0.mm_res]);
+        segs[i].status = b->status.as<int32_t>();
         segs[i].ranked = R.ranked;
         segs[i].block0 = blocks;
         segs[i].nblocks = batch_scan_blocks(R.cap);
@@ -2781,7 +2787,7 @@ int dq_plan_execute(dq_plan* plan, void* stream, dq_result** out) {
       if (attempt >= 8 || (status & (kErrTimeout | kErrBadOp)))
         throw DqError(status & kErrTimeout ? DQ_ERR_TIMEOUT
                       : status & kErrHtFull ? DQ_ERR_HT_FULL
-                      : status & kErrOverflow ? DQ_ERR_OVERFLOW : DQ_ERR_BAD_IR,
+                      : status & (kErrOverflow | kErrMultiFull) ? DQ_ERR_OVERFLOW : DQ_ERR_BAD_IR,
                       "device status " + std::to_string(status));
       // grow what overflowed and run again (the results of a failed run are discarded)
       grow_plan(plan, status);
@@ -3588,6 +3594,8 @@ void srv_dispatch_batch(dq_server* s, SrvSlot& slot, SrvShape* sh) {
         segs[i].counts = R.counts;
         segs[i].ranges = R.ranges;
         segs[i].n = R.cap;
+        segs[i].pay_rows = multi_room(*B.members[i].second->plan->res[S.mm_res]);
+        segs[i].status = B.status.as<int32_t>();
         segs[i].ranked = R.ranked;
         segs[i].block0 = blocks;
         segs[i].nblocks = batch_scan_blocks(R.cap);

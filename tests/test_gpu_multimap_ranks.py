@@ -90,3 +90,49 @@ def test_staged_build_side_outgrows_its_estimate(engine, selectivity):
     plan, cfg = W.plan_c17(alg, scal, Type, Reduction, numgroups=2000)
     cfg = {k: dict(v, selectivity=selectivity) if "selectivity" in v else v for k, v in cfg.items()}
     _check(engine, db, alg.resolveAlgebraPlan(plan, cfg))
+
+
+@pytest.mark.parametrize("prebuilt", [False, True])
+def test_expanding_build_side_outgrows_its_source(engine, prebuilt):
+    """A build side that is itself a multimatch join (and, on generated kernels,
+    carries a string, so that its rows are not staged) has many more rows than
+    the table its pipelines scan: the run ends before a row is placed, the
+    payload grows and the run repeats; alone, in a batch and served."""
+    import dogqc_b200._lib as L
+    from dogqc_b200.database import Database, StringColumn, Table
+    from dogqc_b200.engine import Engine
+    from dogqc_b200.lowering import Lowering
+    from dogqc_b200.relational import Reduction, RelationalAlgebra
+    from dogqc_b200.serve import Server
+    from dogqc_b200.types import Type as T
+    r = np.random.default_rng(3)
+    text = [b"name %d" % (i % 11) + b"x" * (i % 40) for i in range(400)]
+    db = Database([Table("x", {"a": r.integers(0, 10, 400, dtype=np.int32), "s": StringColumn.from_list(text),
+                               "t": r.integers(0, 7, 400, dtype=np.int32)}, {"a": T.INT, "s": T.STRING, "t": T.INT}),
+                   Table("y", {"b": r.integers(0, 10, 500, dtype=np.int32), "c": r.integers(0, 20, 500, dtype=np.int32)},
+                         {"b": T.INT, "c": T.INT}),
+                   Table("p", {"d": r.integers(0, 26, 60, dtype=np.int32)}, {"d": T.INT})])
+    alg = RelationalAlgebra(db)
+    pairs = alg.join(("a", "b"), alg.scan("x"), alg.scan("y"))
+    key = "t" if prebuilt else "s"
+    agg = alg.aggregation([key], [(Reduction.COUNT, "", "n")], alg.join(("c", "d"), pairs, alg.scan("p")))
+    plan = alg.resolveAlgebraPlan(agg, {agg.opId: {"numgroups": 400}})
+    if prebuilt:
+        e = Engine(0, flags=L.CFG_NO_JIT)
+        try:
+            _check(e, db, plan)
+        finally:
+            e.close()
+        return
+    _check(engine, db, plan)
+    want = canonical_rows(run_plan(db, plan)[1])
+    b = engine.prepare_batch([Lowering(plan), Lowering(plan)])
+    for _ in range(2):
+        assert [canonical_rows(res.rows()) for res in b.execute()] == [want, want]
+    b.free()
+    srv = Server(engine, slots=2)
+    try:
+        tickets = [srv.submit(Lowering(plan)) for _ in range(4)]
+        assert [canonical_rows(srv.wait(t)[0].rows()) for t in tickets] == [want] * 4
+    finally:
+        srv.stop()
