@@ -1427,9 +1427,9 @@ struct Gen {
         L("const uint32_t pi_ = id_ * " + num(block) + "u + (uint32_t)tid;");
         for (int j = 0; j < R.naggs; ++j) {
           const bool count = R.agg_red[j] == DQ_RED_COUNT;
-          const std::string T = count ? "uint32_t" : "uint64_t", a = "pa" + num(j) + "_";
+          const std::string T = narrow_count(j) ? "uint32_t" : "uint64_t", a = "pa" + num(j) + "_";
           L(T + "* const " + a + " = reinterpret_cast<" + T + "*>(smem + " + num(priv_at[j]) + ") + pi_;");
-          if (count) L("*" + a + " += 1u;");
+          if (count) L("++*" + a + ";");
           else L("*" + a + " = red_combine(" + red_name(R.agg_red[j]) + ", *" + a + ", " + vals[j] + ");");
         }
         --ind;
@@ -1615,6 +1615,14 @@ struct Gen {
     L("}");
   }
 
+  // Whether a thread's own copy of accumulator j takes 32 bits.
+  bool narrow_count(int j) const {
+    if (P.res[agg_res].agg_red[j] != DQ_RED_COUNT) return false;
+    for (int k = 0; k < P.nops; ++k)
+      if (P.ops[k].kind == DQ_OP_EXPAND) return false;
+    return true;
+  }
+
   // --------------------------------------------------------- aggregation --
   void choose_agg() {
     const dq_op& sink = P.ops[P.nops - 1];
@@ -1636,13 +1644,14 @@ struct Gen {
     // loads and stores where shared atomics return, carry and serialise.  Only
     // up to kPrivateMax: what shared memory takes, the SM's L1 loses for the
     // loads in flight.  (Q1's six groups of six accumulators, 6 M rows: 82 -> 63
-    // us; the same from 16 to 48 warps an SM.)  Counts are 32 bits (a thread
-    // sees fewer rows).  The hint says how many groups to expect;
+    // us; the same from 16 to 48 warps an SM.)  Counts of scanned rows are 32
+    // bits (a thread sees fewer); behind an expansion a thread counts pairs,
+    // which nothing bounds, in 64.  The hint says how many groups to expect;
     // a group beyond it goes to the CTA's one copy beside them.
     if (R.packed && allow_private) {
       const int G = (int)std::min<int64_t>(R.group_hint, kPrivateSlots / 4);
       int row = 0;
-      for (int j = 0; j < R.naggs; ++j) row += R.agg_red[j] == DQ_RED_COUNT ? 4 : 8;
+      for (int j = 0; j < R.naggs; ++j) row += narrow_count(j) ? 4 : 8;
       if (R.group_hint > 0 && R.group_hint <= kPrivateSlots / 4 && G * row * block <= kPrivateMax) {
         agg = AGG_PRIVATE;
         ns = kPrivateSlots;
@@ -1655,7 +1664,7 @@ struct Gen {
         priv_at.assign(R.naggs, 0);
         for (int pass = 0; pass < 2; ++pass)  // 64-bit accumulators first
           for (int j = 0; j < R.naggs; ++j)
-            if ((R.agg_red[j] == DQ_RED_COUNT) == (pass == 1)) {
+            if (narrow_count(j) == (pass == 1)) {
               priv_at[j] = smem;
               smem += G * block * (pass == 1 ? 4 : 8);
             }
@@ -2016,7 +2025,7 @@ struct Gen {
       L("uint32_t* const lids = reinterpret_cast<uint32_t*>(smem + " + num(priv_id_off) + ");  // group numbers, then their count");
       L("for (int i = tid; i <= " + num(ns + 1) + "; i += " + num(block) + ") lids[i] = i <= " + num(ns) + " ? kEmpty32 : 0u;");
       for (int j = 0; j < R.naggs; ++j) {
-        const bool count = R.agg_red[j] == DQ_RED_COUNT;
+        const bool count = narrow_count(j);
         const std::string T = count ? "uint32_t" : "uint64_t";
         L("for (int i = tid; i < " + num(priv * block) + "; i += " + num(block) + ") reinterpret_cast<" + T + "*>(smem + " +
           num(priv_at[j]) + ")[i] = " + (count ? std::string("0u") : std::string("red_init(") + red_name(R.agg_red[j]) + ")") + ";");
@@ -2052,8 +2061,7 @@ struct Gen {
       L("switch (j_) {");
       ++ind;
       for (int j = 0; j < R.naggs; ++j) {
-        const bool count = R.agg_red[j] == DQ_RED_COUNT;
-        const std::string T = count ? "uint32_t" : "uint64_t", red = red_name(R.agg_red[j]);
+        const std::string T = narrow_count(j) ? "uint32_t" : "uint64_t", red = red_name(R.agg_red[j]);
         L("case " + num(j) + ": {");
         ++ind;
         L("const " + T + "* const a_ = reinterpret_cast<const " + T + "*>(smem + " + num(priv_at[j]) + ") + id_ * " + num(block) +

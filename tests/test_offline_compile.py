@@ -173,3 +173,25 @@ def test_like_patterns_of_percent_separated_literals_compile_to_searches(engine,
     body = src[src.index("dq_main"):]
     assert ("like_find(" in body) == search
     assert ("like_match(" in body) == (not search)
+
+
+@pytest.mark.parametrize("expands", [False, True])
+def test_private_counts_hold_pairs(engine, expands):
+    """Threads count scanned rows in 32 bits and, behind an expansion, pairs
+    (which no table's size bounds) in 64."""
+    import numpy as np
+    from dogqc_b200.database import Database, Table
+    from dogqc_b200.relational import Reduction
+    from dogqc_b200.types import Type
+    n = np.arange(1000, dtype=np.int32)
+    db = Database([Table("b", {"k": n % 50}, {"k": Type.INT}),
+                   Table("p", {"q": n % 60, "g": n % 4}, {"q": Type.INT, "g": Type.INT})])
+    engine.register_database(db, force=True)
+    alg = RelationalAlgebra(db)
+    rows = alg.join(("k", "q"), alg.scan("b"), alg.scan("p")) if expands else alg.scan("p")
+    agg = alg.aggregation(["g"], [(Reduction.COUNT, "", "n")], rows)
+    plan = engine.prepare(alg.resolveAlgebraPlan(agg, {agg.opId: {"numgroups": 4}}))
+    src = [plan.source(i) for i in range(len(plan.lowering.pipes))]
+    src = [s for s in src if "pa0_" in s][0]
+    assert ("uint64_t* const pa0_" in src, "uint32_t* const pa0_" in src) == (expands, not expands)
+    check_sources(plan)
