@@ -1370,7 +1370,8 @@ int enqueue_run(dq_plan* plan, cudaStream_t st, int32_t* host_status, bool fast 
     }
     dag = forks;
   }
-  auto lane_stream = [&](int l) { return l == 0 ? st : plan->lanes[(size_t)l - 1]; };
+  const cudaStream_t origin = st;  // (`st` moves from lane to lane below)
+  auto lane_stream = [&](int l) { return l == 0 ? origin : plan->lanes[(size_t)l - 1]; };
   if (plan->events.size() != 2 * np + 2) {
     free_events(plan);
     for (size_t i = 0; i < 2 * np + 2; ++i) {
@@ -1385,7 +1386,6 @@ int enqueue_run(dq_plan* plan, cudaStream_t st, int32_t* host_status, bool fast 
   launches += enqueue_resets(plan, st);
   for (auto& rp : plan->res) rp->agg_clean = false;
   if (dag) DQ_CUDA(cudaEventRecord(plan->fork_ev, st));
-  const cudaStream_t origin = st;
   uint32_t* counters = plan->counters;
   for (size_t i = 0; i < np; ++i) {
     PipeRec& p = *plan->pipes[i];

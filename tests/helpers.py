@@ -43,3 +43,33 @@ def result_checksum(rows, spec):
     if spec.get("str_cols"):
         return canonical_checksum(reference_rows(rows, spec))
     return canonical_checksum(rows)
+
+
+def many_domains(dims, keys, groups=11, rows=20_000):
+    """A filtered fact table semi-joined with ``dims`` dimensions of ``keys``
+    keys each (a key bitmap a dimension), summed by ``groups`` groups."""
+    import numpy as np
+    import dogqc_b200.scalar as scal
+    from dogqc_b200.database import Database, Table
+    from dogqc_b200.relational import Reduction
+    from dogqc_b200.types import Type
+    r = np.random.default_rng(dims)
+    fact = {"g": r.integers(0, groups, rows, dtype=np.int32), "v": r.integers(0, 1 << 30, rows).astype(np.uint64),
+            "f": r.integers(0, 100, rows, dtype=np.int32)}
+    tables = []
+    for i in range(dims):
+        k = r.permutation(keys)[:keys * 3 // 4].astype(np.int32)
+        k[:2] = (0, keys - 1)
+        tables.append(Table("d%d" % i, {"k%d" % i: k}, {"k%d" % i: Type.INT}))
+        fact["q%d" % i] = r.integers(0, keys, rows, dtype=np.int32)
+    tables.append(Table("fact", fact, {c: Type.FLOAT if c == "v" else Type.INT for c in fact}))
+    db = Database(tables)
+    alg = RelationalAlgebra(db)
+    node = alg.selection(scal.SmallerExpr(scal.AttrExpr("f"), scal.ConstExpr("40", Type.INT)), alg.scan("fact"))
+    cfg = {node.opId: {"selectivity": 0.4}}
+    for i in range(dims):
+        node = alg.semijoin(("k%d" % i, "q%d" % i), None, alg.scan("d%d" % i), node)
+        cfg[node.opId] = {"multimatch": False, "selectivity": 0.75}
+    agg = alg.aggregation(["g"], [(Reduction.SUM, "v", "s")], node)
+    cfg[agg.opId] = {"numgroups": groups}
+    return db, alg.resolveAlgebraPlan(agg, cfg)
