@@ -45,6 +45,8 @@ namespace {
 
 constexpr int kStripedMax = 12 * 1024;      // shared memory a replicated CTA-local aggregation table may take
 constexpr int kPrivateMax = 68 * 1024;      // shared memory per-thread accumulators of a CTA may take
+constexpr int kSmemMax = 227 * 1024 - 2048; // shared memory of a CTA beside the kernels' static arrays
+constexpr int kFrugal = 4;                  // see Gen::frugal
 constexpr int kPrivateSlots = 64;           // group slots beside them
 constexpr int kBlock = kThreads;
 constexpr int kTailChunk = 8;               // slots a thread of a fused tail looks at together
@@ -182,15 +184,18 @@ struct Gen {
   int ns = 0;                    // local table slots (without the all-ones slot)
   int copies = 1;
   int priv = 0;                  // AGG_PRIVATE: groups with accumulators per thread
-  int priv_off = 0;              // shared-memory offset of those (accumulator j's from priv_at[j])
+  std::vector<int> priv_at;      // shared-memory offsets of those, by accumulator
   int priv_id_off = 0;           // and of the slots' group numbers
-  std::vector<int> priv_at;
   int U = 1;
   int smem = 0;
   std::string pay_reg;           // probe payload already loaded with its tag
   std::vector<int> prefetch;     // probes whose first slot pair is loaded early
   std::map<int, std::string> pending;  // gathered slots not loaded yet -> match index
-  bool allow_private = true;     // per-thread accumulators may be chosen
+  int frugal = 0;                // what a kernel whose CTA would need more shared memory
+                                 // than there is gives up: from 1 the accumulators per
+                                 // thread, from 2 CTAs of more than kBlock threads, from 3
+                                 // bits of its own and of multimaps, at kFrugal (4) staged key
+                                 // bitmaps that do not fit
   int min_blocks = 0;            // __launch_bounds__ minimum CTAs per SM (0: none)
   int refill = -1;               // op after which lanes are refilled (-1: none)
   int refill_threshold = 32;     // buffered rows that make the warp process them
@@ -1648,7 +1653,7 @@ struct Gen {
     // bits (a thread sees fewer); behind an expansion a thread counts pairs,
     // which nothing bounds, in 64.  The hint says how many groups to expect;
     // a group beyond it goes to the CTA's one copy beside them.
-    if (R.packed && allow_private) {
+    if (R.packed && frugal < 1) {
       const int G = (int)std::min<int64_t>(R.group_hint, kPrivateSlots / 4);
       int row = 0;
       for (int j = 0; j < R.naggs; ++j) row += narrow_count(j) ? 4 : 8;
@@ -1660,7 +1665,6 @@ struct Gen {
         smem = (ns + 1) * 8 * (1 + R.naggs);
         priv_id_off = smem;
         smem = (smem + (ns + 2) * 4 + 15) / 16 * 16;
-        priv_off = smem;
         priv_at.assign(R.naggs, 0);
         for (int pass = 0; pass < 2; ++pass)  // 64-bit accumulators first
           for (int j = 0; j < R.naggs; ++j)
@@ -1758,7 +1762,7 @@ struct Gen {
   // the table's rows say little about the pairs.
   void choose_own_bits() {
     bits_off = -1;
-    if (batched || P.nops == 0 || P.source_kind != DQ_SRC_TABLE) return;
+    if (frugal >= 3 || batched || P.nops == 0 || P.source_kind != DQ_SRC_TABLE) return;
     for (int j = 0; j < P.nops; ++j)
       if (P.ops[j].kind == DQ_OP_EXPAND) return;
     const dq_op& sink = P.ops[P.nops - 1];
@@ -2139,7 +2143,7 @@ struct Gen {
       if (op.kind == DQ_OP_PROBE && P.res[op.res].bitmap == 1) {
         words = (long long)P.res[op.res].cap;
         bits = "reinterpret_cast<const uint32_t*>(" + res(op.res) + ".slots)";
-      } else if ((op.kind == DQ_OP_EXPAND || op.kind == DQ_OP_EXISTS) && P.res[op.res].filter) {
+      } else if ((op.kind == DQ_OP_EXPAND || op.kind == DQ_OP_EXISTS) && P.res[op.res].filter && frugal < 3) {
         words = ((long long)P.res[op.res].brange + 31) / 32;
         bits = res(op.res) + ".bits";
       }
@@ -2148,6 +2152,7 @@ struct Gen {
       for (auto& b : bitmaps) seen |= b.res == op.res;
       if (seen) continue;
       const int off = (smem + 15) / 16 * 16;
+      if (frugal >= kFrugal && off + words * 4 > kSmemMax) continue;
       bitmaps.push_back({op.res, off, words, bits});
       smem = off + (int)words * 4;
     }
@@ -2688,13 +2693,16 @@ struct Gen {
 
 }  // namespace
 
-Program generate(const DevPipe& P, int expand_op, int refill_op, const Tuning& t, const DevPipe* tail,
-                 const std::string* patterns) {
+// The generator for a pipeline, with its choices of launch shape, tables and
+// shared memory made.
+static Gen choose(const DevPipe& P, int expand_op, int refill_op, const Tuning& t, const std::string* patterns,
+                  int frugal) {
   Gen g(P, expand_op);
   g.patterns = patterns;
   g.batched = t.batched;
+  g.frugal = frugal;
   if (t.block == 128 || t.block == 256 || t.block == 512) g.block = t.block;
-  else if (!t.batched && g.staged_bits() >= kWideBits) g.block = 512, g.min_blocks = 2;
+  else if (!t.batched && frugal < 2 && g.staged_bits() >= kWideBits) g.block = 512, g.min_blocks = 2;
   if (t.min_blocks > 0 && t.min_blocks * g.block <= 2048) g.min_blocks = t.min_blocks;
   bool has_expand = false;
   for (int i = 0; i < P.nops; ++i) has_expand |= P.ops[i].kind == DQ_OP_EXPAND;
@@ -2718,7 +2726,7 @@ Program generate(const DevPipe& P, int expand_op, int refill_op, const Tuning& t
   // group and accumulator on the same few addresses as every other CTA: twice
   // the threads a CTA, half the merges (6 M probes into 25 groups of two, 256
   // threads 49.8 us, 512 43.3)
-  if (g.agg == AGG_STRIPED && P.res[g.agg_res].packed && t.block == 0 && !t.batched) g.block = 512;
+  if (g.agg == AGG_STRIPED && P.res[g.agg_res].packed && t.block == 0 && !t.batched && frugal < 2) g.block = 512;
   g.choose_refill(refill_op);
   g.choose_hot();
   g.choose_own_bits();
@@ -2733,6 +2741,16 @@ Program generate(const DevPipe& P, int expand_op, int refill_op, const Tuning& t
         cols.push_back(P.slots[s].src);
     if ((cols.size() > 3 && g.agg != AGG_PRIVATE) || g.prefetch.size() > 1) g.U = 2;
   }
+  return g;
+}
+
+Program generate(const DevPipe& P, int expand_op, int refill_op, const Tuning& t, const DevPipe* tail,
+                 const std::string* patterns) {
+  // Each choice is made for itself; together they may pass what a CTA has (four
+  // probed domains of 2^18 keys beside eleven groups: 249,632 bytes).
+  int frugal = 0;
+  while (frugal < kFrugal && choose(P, expand_op, refill_op, t, patterns, frugal).smem > kSmemMax) ++frugal;
+  Gen g = choose(P, expand_op, refill_op, t, patterns, frugal);
   g.o = "// generated pipeline kernel (dogqc_b200)\n#include \"dq_common.cuh\"\nusing namespace dq;\n\n";
   if (tail && !t.batched && expand_op < 0) {
     Gen tg(*tail, -1);

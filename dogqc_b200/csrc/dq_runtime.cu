@@ -257,6 +257,7 @@ struct ColRec {
   uint64_t nchars = 0;
   std::shared_ptr<DevBuf> data;
   std::shared_ptr<DevBuf> offsets;
+  long long lo = LLONG_MAX, hi = LLONG_MIN;  // offline contexts: an integer column's values
 };
 
 struct TableRec {
@@ -489,10 +490,28 @@ int guarded(dq_ctx* ctx, F f) {
   }
 }
 
+// The smallest and largest value of an integer column in host memory.
+void host_range(ColRec& rec, const dq_column& c, int64_t nrows) {
+  rec.lo = LLONG_MAX, rec.hi = LLONG_MIN;
+  auto scan = [&](auto* v) {
+    for (int64_t i = 0; i < nrows; ++i) {
+      rec.lo = std::min(rec.lo, (long long)v[i]);
+      rec.hi = std::max(rec.hi, (long long)v[i]);
+    }
+  };
+  switch (c.ctype) {
+    case DQ_I8: return scan(static_cast<const int8_t*>(c.data));
+    case DQ_I32: return scan(static_cast<const int32_t*>(c.data));
+    case DQ_U32: return scan(static_cast<const uint32_t*>(c.data));
+    case DQ_I64: return scan(static_cast<const int64_t*>(c.data));
+  }
+}
+
 void upload_column(dq_ctx* ctx, ColRec& rec, const dq_column& c, int64_t nrows, bool device_src,
                    cudaStream_t stream) {
   cudaMemcpyKind kind = device_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  if (ctx->offline) {  // sizes only
+  if (ctx->offline) {  // sizes and value ranges only
+    if (!device_src) host_range(rec, c, nrows);
     if (!rec.data) rec.data = std::make_shared<DevBuf>();
     if (c.ctype == DQ_STR && c.width <= 0 && !rec.offsets) rec.offsets = std::make_shared<DevBuf>();
     return;
@@ -784,6 +803,13 @@ void validate_pipeline(const dq_pipeline& d, int nres) {
         (sl.res < 0 || sl.res >= nres))
       throw DqError(DQ_ERR_BAD_IR, "slot resource out of range");
   }
+}
+
+// A generated kernel's shared memory against what a CTA may have.
+void check_smem(const jit::Program& prog) {
+  if (prog.smem_bytes > 227 * 1024)
+    throw DqError(DQ_ERR_UNSUPPORTED, "a pipeline needs " + std::to_string(prog.smem_bytes) +
+                                          " bytes of shared memory, more than a CTA has");
 }
 
 void setup_pipeline(dq_plan* plan, PipeRec& p) {
@@ -1097,6 +1123,7 @@ void setup_pipeline(dq_plan* plan, PipeRec& p) {
     const DevPipe* tail = p.tail >= 0 && p.expand_op < 0 ? &plan->pipes[p.tail]->dev : nullptr;
     if (p.tail >= 0 && !tail) throw DqError(DQ_ERR_BAD_IR, "a pipeline with deferred expansion cannot run a fused tail");
     p.prog = jit::generate(P, p.expand_op, d.compact - 1, plan->opts.tuning, tail, &p.pattern_text);
+    check_smem(p.prog);
     if (t_collect) t_collect->push_back(p.prog);
     else p.kernels = jit::compile(p.prog, !ctx->offline);
     rows_per_cta = (int64_t)p.prog.block * p.prog.rows_per_thread;
@@ -1728,6 +1755,10 @@ bool fusable_tail(const dq_plan_desc* desc, const std::vector<std::unique_ptr<Re
 
 // The smallest and largest value of an integer column (false: no rows).
 bool column_range(dq_ctx* ctx, const ColRec& c, uint64_t rows, long long* got) {
+  if (ctx->offline) {
+    got[0] = c.lo, got[1] = c.hi;
+    return c.lo <= c.hi;
+  }
   DevBuf mm;
   mm.alloc(16);
   const long long init[2] = {LLONG_MAX, LLONG_MIN};
@@ -1787,7 +1818,7 @@ void choose_bitmap(dq_ctx* ctx, const dq_plan_desc* desc, int i, ResRec& r) {
   if (t == ctx->tables.end() || t->second.nrows <= 0) return;
   const ColRec* c = t->second.find(build->cols[ci]);
   // the key is the column's value unchanged: same type in the slot and the table
-  if (!c || c->ctype != kt || build->slots[ks].ctype != kt || !c->data || !c->data->ptr) return;
+  if (!c || c->ctype != kt || build->slots[ks].ctype != kt || !c->data || !(c->data->ptr || ctx->offline)) return;
   long long got[2];
   if (!column_range(ctx, *c, (uint64_t)t->second.nrows, got)) return;
   const uint64_t span = (uint64_t)got[1] - (uint64_t)got[0] + 1;  // 0: all 2^64 values
@@ -1825,7 +1856,7 @@ void choose_filter(dq_ctx* ctx, const dq_plan_desc* desc, int i, ResRec& r) {
   auto t = ctx->tables.find(build->table);
   if (t == ctx->tables.end() || t->second.nrows <= 0) return;
   const ColRec* c = t->second.find(build->cols[ci]);
-  if (!c || c->ctype != kt || build->slots[ks].ctype != kt || !c->data || !c->data->ptr) return;
+  if (!c || c->ctype != kt || build->slots[ks].ctype != kt || !c->data || !(c->data->ptr || ctx->offline)) return;
   if (d.capacity * 4 > t->second.nrows) return;
   long long got[2];
   if (!column_range(ctx, *c, (uint64_t)t->second.nrows, got)) return;
@@ -1895,11 +1926,12 @@ std::unique_ptr<dq_plan> make_plan(dq_ctx* ctx, const dq_plan_desc* desc, const 
     r->desc = desc->res[i];
     r->name = desc->res[i].name ? desc->res[i].name : "";
     r->desc.name = nullptr;
-    if (!(ctx->cfg.flags & (DQ_CFG_NO_JIT | DQ_CFG_ROW_KERNEL)) && !ctx->offline && !t_offline)
+    const bool measured = ctx->offline || !t_offline;  // the columns' value ranges can be had
+    if (!(ctx->cfg.flags & (DQ_CFG_NO_JIT | DQ_CFG_ROW_KERNEL)) && measured)
       choose_bitmap(ctx, desc, i, *r);
     r->ranked = r->desc.kind == DQ_RES_MULTI && ranked[i] && built[i] >= 0;
     r->src_rows = (uint64_t)bound[i];
-    if (r->ranked && !ctx->offline && !t_offline && !opts.batch_member) choose_filter(ctx, desc, i, *r);
+    if (r->ranked && measured && !opts.batch_member) choose_filter(ctx, desc, i, *r);
     setup_resource(plan.get(), *r, bound[i]);
     plan->res.push_back(std::move(r));
   }
@@ -2175,6 +2207,7 @@ void build_batch(dq_batch* b, const jit::Tuning& tuning, cudaStream_t st) {
           jit::generate(pi.dev, pi.expand_op, pi.desc.compact - 1, t).source != S.prog.source)
         throw DqError(DQ_ERR_BAD_IR, "batch instance " + std::to_string(i) + " differs in shape from instance 0");
     }
+    check_smem(S.prog);
     S.kernels = jit::compile(S.prog, !ctx->offline);
     if (ctx->offline) continue;
     if (p0.expand_op >= 0) setup_batch_heavy(b, p, S);

@@ -75,3 +75,16 @@ def test_keys_leaving_the_domain_fall_back_to_a_hash_table(engine):
         assert not _bitmap_pipelines(p)
     finally:
         p.free()
+
+
+@pytest.mark.parametrize("dims", [1, 3, 4, 5, 8])
+def test_many_domains(engine, dims):
+    """More staged bitmaps than a CTA has room for beside its other tables."""
+    from helpers import many_domains
+    db, plan = many_domains(dims, 1 << 18)
+    engine.register_database(db, force=True)
+    p = engine.prepare(plan)
+    want = canonical_rows(run_plan(db, plan)[1])
+    for _ in range(2):
+        assert canonical_rows(p.execute().rows()) == want
+    p.free()

@@ -195,3 +195,17 @@ def test_private_counts_hold_pairs(engine, expands):
     src = [s for s in src if "pa0_" in s][0]
     assert ("uint64_t* const pa0_" in src, "uint32_t* const pa0_" in src) == (expands, not expands)
     check_sources(plan)
+
+
+@pytest.mark.parametrize("dims", [1, 4, 5, 8])
+def test_shared_memory_has_a_budget(engine, dims):
+    """Staged key bitmaps, accumulators per thread and refill buffers together
+    stay within what a CTA has: a kernel gives some of them up."""
+    from helpers import many_domains
+    db, resolved_plan = many_domains(dims, 1 << 18)
+    engine.register_database(db, force=True)
+    plan = engine.prepare(resolved_plan)
+    check_sources(plan)
+    fact = [plan.source(i) for i in range(dims, len(plan.lowering.pipes))][0]
+    assert ("pa0_" in fact) == (dims <= 4)                  # accumulators per thread
+    assert fact.count("= __ldcg(g_ + i)") == min(dims, 5)   # staged bitmaps
