@@ -85,9 +85,11 @@ struct DqError : std::runtime_error {
 #define DQ_CUDA(expr)                                                                        \
   do {                                                                                       \
     cudaError_t _e = (expr);                                                                 \
-    if (_e != cudaSuccess)                                                                   \
+    if (_e != cudaSuccess) {                                                                 \
+      cudaGetLastError(); /* reported here: the next call's launches must not find it */     \
       throw DqError(_e == cudaErrorMemoryAllocation ? DQ_ERR_OOM : DQ_ERR_CUDA,              \
                     std::string(#expr) + ": " + cudaGetErrorString(_e));                     \
+    }                                                                                        \
   } while (0)
 
 int ctype_width(int t) {
