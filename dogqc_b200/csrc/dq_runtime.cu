@@ -166,44 +166,64 @@ struct DevBuf {
 };
 
 // Pinned blocks that large results are copied into, lent to a result and given
-// back when it is freed.  At most kPoolIdle bytes stay unused in the pool.  The
-// context and the results share it: a result may outlive its context.
-constexpr size_t kPoolIdle = 64ull << 20;
+// back when it is freed.  The pool holds at most kPoolBytes, lent blocks
+// included: a result past that takes ordinary memory, since pinning and
+// unpinning a block costs more than one copy saves (5 M rows of 12 bytes: 46 ms
+// a pass with a 64 MB block pinned each time, 30 in ordinary memory, 11 in blocks
+// that stay; 12 M rows: 101, 88 and, half of them in such blocks, 75).
+// The context and the results share the pool: a result may outlive its context.
+constexpr size_t kPoolBytes = 64ull << 20;
 constexpr size_t kPoolLeast = 64ull << 10;  // smaller columns take ordinary memory
 struct PinnedPool {
   std::mutex mu;
   std::multimap<size_t, void*> idle;  // by block size
-  size_t idle_bytes = 0;
+  size_t held = 0;                    // bytes of all blocks, idle and lent
   ~PinnedPool() {
     for (auto& b : idle) cudaFreeHost(b.second);
   }
+  // A block of at least `bytes` (its size in `block`), or nullptr: an idle one
+  // of a like size, else a new one, else any idle one that is large enough; idle
+  // ones that are all too small make room for it.
   void* take(size_t bytes, size_t& block) {
+    const size_t step = bytes < (1 << 20) ? kPoolLeast : 1 << 20;
+    const size_t fresh = (bytes + step - 1) / step * step;
+    std::vector<void*> drop;
     {
       std::lock_guard<std::mutex> lk(mu);
       auto it = idle.lower_bound(bytes);
-      if (it != idle.end() && it->first <= 4 * bytes) {
+      if (it != idle.end() && (it->first <= 4 * bytes || held + fresh > kPoolBytes)) {
         void* p = it->second;
         block = it->first;
-        idle_bytes -= block;
         idle.erase(it);
         return p;
       }
-    }
-    block = kPoolLeast;
-    while (block < bytes) block *= 2;
-    void* p = nullptr;
-    return cudaMallocHost(&p, block) == cudaSuccess ? p : nullptr;
-  }
-  void give(void* p, size_t block) {
-    {
-      std::lock_guard<std::mutex> lk(mu);
-      if (idle_bytes + block <= kPoolIdle) {
-        idle.emplace(block, p);
-        idle_bytes += block;
-        return;
+      size_t unused = 0;
+      for (auto& b : idle) unused += b.first;
+      if (held - unused + fresh > kPoolBytes) return nullptr;
+      while (held + fresh > kPoolBytes) {
+        held -= idle.begin()->first;
+        drop.push_back(idle.begin()->second);
+        idle.erase(idle.begin());
       }
+      held += fresh;
     }
-    cudaFreeHost(p);
+    for (void* p : drop) cudaFreeHost(p);
+    void* p = nullptr;
+    block = fresh;
+    if (cudaMallocHost(&p, fresh) == cudaSuccess) return p;
+    cudaGetLastError();
+    std::lock_guard<std::mutex> lk(mu);
+    held -= fresh;
+    return nullptr;
+  }
+  void give(void* p, size_t block) noexcept {
+    std::lock_guard<std::mutex> lk(mu);
+    try {
+      idle.emplace(block, p);
+    } catch (...) {  // no memory for the entry
+      held -= block;
+      cudaFreeHost(p);
+    }
   }
 };
 
@@ -236,7 +256,6 @@ class HostBytes {
     if (pool && n >= kPoolLeast) {
       fresh.p_ = static_cast<uint8_t*>(pool->take(n, fresh.block_));
       if (fresh.p_) fresh.pool_ = pool;
-      else cudaGetLastError();  // no pinned memory: ordinary memory does
     }
     if (!fresh.p_) fresh.p_ = new uint8_t[n ? n : 1];
     swap(fresh);

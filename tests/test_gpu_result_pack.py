@@ -54,3 +54,55 @@ def test_results_outlive_their_plan_and_context():
     engine.close()
     for r in results:
         assert sorted(r.rows()) == expect
+
+
+def test_pinned_memory_of_large_results_is_bounded():
+    """Results of a replaying plan lie in pinned blocks up to 64 MB in all, lent
+    and idle; what goes past that lies in ordinary memory and is as exact."""
+    import ctypes as C
+    from cuda.bindings import runtime as cudart
+    from dogqc_b200 import _lib as L
+    from dogqc_b200.database import Database, Table
+    from dogqc_b200.engine import Engine
+    from dogqc_b200.relational import RelationalAlgebra
+    from dogqc_b200.types import Type
+    n = 3_000_000
+    cols = {"k": np.arange(n, dtype=np.int32), "v": np.random.default_rng(1).integers(0, 1 << 62, n).astype(np.uint64)}
+    db = Database([Table("t", cols, {"k": Type.INT, "v": Type.FLOAT})])
+    alg = RelationalAlgebra(db)
+    e = Engine(0)
+    e.register_database(db)
+    p = e.prepare(alg.resolveAlgebraPlan(alg.projection(["k", "v"], alg.scan("t")), {}))
+    lib = L.lib()
+
+    def run():
+        res = C.c_void_p()
+        L.check(lib.dq_plan_execute(p.handle, None, C.byref(res)), e.ctx)
+        rows, ncols, view = C.c_int64(), C.c_int32(), (L.dq_result_col * L.MAX_PAY)()
+        L.check(lib.dq_result_view(res, C.byref(rows), C.byref(ncols), view))
+        assert rows.value == n and ncols.value == 2
+        pinned = 0
+        got = []
+        for j, dt in enumerate((np.int32, np.uint64)):
+            err, at = cudart.cudaPointerGetAttributes(view[j].data)
+            pinned += view[j].bytes if at.type == cudart.cudaMemoryType.cudaMemoryTypeHost else 0
+            got.append(np.frombuffer((C.c_uint8 * view[j].bytes).from_address(view[j].data), dt))
+        order = np.argsort(got[0])
+        assert (got[0][order] == cols["k"]).all() and (got[1][order] == cols["v"]).all()
+        return res, pinned
+
+    try:
+        for _ in range(2):
+            p.execute()
+        for _ in range(2):  # four results held at once: 144 MB
+            held = [run() for _ in range(4)]
+            assert 0 < sum(b for _, b in held) <= 64 << 20
+            for res, _ in held:
+                lib.dq_result_free(res)
+        for _ in range(3):  # one at a time: all of it pinned
+            res, pinned = run()
+            assert pinned == n * 12
+            lib.dq_result_free(res)
+    finally:
+        p.free()
+        e.close()
