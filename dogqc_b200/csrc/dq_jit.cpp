@@ -210,8 +210,7 @@ struct Gen {
   std::string ldfn = "__ldcs";   // load function of streamed source columns
   struct Staged {                // key-domain bits a CTA holds in shared memory
     int res, off;
-    long long words;
-    std::string bits;            // where they are in global memory
+    std::string words, bits;     // how many there are, and where in global memory
   };
   std::vector<Staged> bitmaps;
   const std::string* patterns = nullptr;     // host copy of the pattern bytes (P.pat_off into it)
@@ -1775,8 +1774,8 @@ struct Gen {
 
   void own_bits_init() {
     if (bits_off < 0) return;
-    const std::string W = num((long long)P.res[P.ops[P.nops - 1].res].cap);
-    L("for (int i = tid; i < " + W + "; i += " + num(block) + ") reinterpret_cast<uint32_t*>(smem + " + num(bits_off) + ")[i] = 0u;");
+    const std::string W = "(uint32_t)" + res(P.ops[P.nops - 1].res) + ".cap";
+    L("for (uint32_t i = tid; i < " + W + "; i += " + num(block) + "u) reinterpret_cast<uint32_t*>(smem + " + num(bits_off) + ")[i] = 0u;");
     L("__syncthreads();");
   }
 
@@ -1784,7 +1783,7 @@ struct Gen {
     if (bits_off < 0) return;
     const int r = P.ops[P.nops - 1].res;
     L("__syncthreads();");
-    L("for (int i = tid; i < " + num((long long)P.res[r].cap) + "; i += " + num(block) + ") {");
+    L("for (uint32_t i = tid; i < (uint32_t)" + res(r) + ".cap; i += " + num(block) + "u) {");
     L("  const uint32_t b_ = reinterpret_cast<const uint32_t*>(smem + " + num(bits_off) + ")[i];");
     L("  if (b_) atomicOr(reinterpret_cast<unsigned int*>(" + res(r) + ".slots) + i, b_);");
     L("}");
@@ -2130,8 +2129,9 @@ struct Gen {
     return bytes;
   }
 
-  // The key-domain bitmaps of at most 32 KB this kernel probes, one word per
-  // thread into shared memory (a probe is then a bank access, not an L2
+  // The key-domain bitmaps of at most 32 KB this kernel probes (their sizes from
+  // the descriptor: plans over tables of other key ranges share the kernel), one
+  // word per thread into shared memory (a probe is then a bank access, not an L2
   // access); larger ones are probed in place.
   void choose_bitmaps() {
     bitmaps.clear();
@@ -2139,12 +2139,14 @@ struct Gen {
     for (int k = 0; k < P.nops; ++k) {
       const dq_op& op = P.ops[k];
       long long words = 0;
-      std::string bits;
+      std::string count, bits;
       if (op.kind == DQ_OP_PROBE && P.res[op.res].bitmap == 1) {
         words = (long long)P.res[op.res].cap;
+        count = "(uint32_t)" + res(op.res) + ".cap";
         bits = "reinterpret_cast<const uint32_t*>(" + res(op.res) + ".slots)";
       } else if ((op.kind == DQ_OP_EXPAND || op.kind == DQ_OP_EXISTS) && P.res[op.res].filter && frugal < 3) {
         words = ((long long)P.res[op.res].brange + 31) / 32;
+        count = "(uint32_t)((" + res(op.res) + ".brange + 31) / 32)";
         bits = res(op.res) + ".bits";
       }
       if (words <= 0 || words > 8192) continue;
@@ -2153,7 +2155,7 @@ struct Gen {
       if (seen) continue;
       const int off = (smem + 15) / 16 * 16;
       if (frugal >= kFrugal && off + words * 4 > kSmemMax) continue;
-      bitmaps.push_back({op.res, off, words, bits});
+      bitmaps.push_back({op.res, off, count, bits});
       smem = off + (int)words * 4;
     }
   }
@@ -2163,7 +2165,7 @@ struct Gen {
       L("{");
       L("  const uint32_t* g_ = " + b.bits + ";");
       L("  uint32_t* s_ = reinterpret_cast<uint32_t*>(smem + " + num(b.off) + ");");
-      L("  for (uint32_t i = tid; i < " + num(b.words) + "u; i += " + num(block) + "u) s_[i] = __ldcg(g_ + i);");
+      L("  for (uint32_t i = tid; i < " + b.words + "; i += " + num(block) + "u) s_[i] = __ldcg(g_ + i);");
       L("}");
     }
     if (!bitmaps.empty()) L("__syncthreads();");

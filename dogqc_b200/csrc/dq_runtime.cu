@@ -833,6 +833,18 @@ void check_smem(const jit::Program& prog) {
                                           " bytes of shared memory, more than a CTA has");
 }
 
+// Lets a kernel be launched with `bytes` of shared memory.  Plans share kernels
+// and need not agree on the bytes (staged bitmaps of other domains), so the
+// kernel's limit only ever grows.
+void allow_smem(const void* fn, int bytes) {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  cudaFuncAttributes a;
+  DQ_CUDA(cudaFuncGetAttributes(&a, fn));
+  if (a.maxDynamicSharedSizeBytes < bytes)
+    DQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+}
+
 void setup_pipeline(dq_plan* plan, PipeRec& p) {
   dq_ctx* ctx = plan->ctx;
   const dq_pipeline& d = p.desc;
@@ -1150,11 +1162,9 @@ void setup_pipeline(dq_plan* plan, PipeRec& p) {
     rows_per_cta = (int64_t)p.prog.block * p.prog.rows_per_thread;
     if (!ctx->offline && !t_offline) {
       const void* fn = (const void*)p.kernels.main;
-      DQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, p.prog.smem_bytes));
+      allow_smem(fn, p.prog.smem_bytes);
       DQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, p.prog.block, p.prog.smem_bytes));
-      if (p.kernels.heavy)
-        DQ_CUDA(cudaFuncSetAttribute((const void*)p.kernels.heavy, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     p.prog.smem_bytes));
+      if (p.kernels.heavy) allow_smem((const void*)p.kernels.heavy, p.prog.smem_bytes);
     }
   } else if (!ctx->offline) {
     occ = p.row ? row_occupancy(P.smem_bytes) : pipeline_occupancy(P.smem_bytes);
@@ -2254,14 +2264,14 @@ void build_batch(dq_batch* b, const jit::Tuning& tuning, cudaStream_t st) {
     upload(S.descs, descs);
     upload(S.bprefix, prefix);
     const void* fn = (const void*)S.kernels.main;
-    DQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S.prog.smem_bytes));
+    allow_smem(fn, S.prog.smem_bytes);
     int occ = 0;
     DQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, S.prog.block, S.prog.smem_bytes));
     if (occ < 1) throw DqError(DQ_ERR_UNSUPPORTED, "batched pipeline kernel cannot be resident");
     S.grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->sms * occ, prefix[b->ninst]));
     if (S.kernels.heavy) {
       const void* hf = (const void*)S.kernels.heavy;
-      DQ_CUDA(cudaFuncSetAttribute(hf, cudaFuncAttributeMaxDynamicSharedMemorySize, S.prog.smem_bytes));
+      allow_smem(hf, S.prog.smem_bytes);
       int hocc = 0;
       DQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&hocc, hf, S.prog.block, S.prog.smem_bytes));
       S.heavy_grid = ctx->sms * std::max(hocc, 1);
@@ -3539,11 +3549,11 @@ SrvShape* srv_shape(dq_server* s, dq_plan* plan) {
     st.prog = progs[p];
     st.kernels = jit::compile(st.prog, true);
     const void* fn = (const void*)st.kernels.main;
-    DQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, st.prog.smem_bytes));
+    allow_smem(fn, st.prog.smem_bytes);
     DQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&st.occ, fn, st.prog.block, st.prog.smem_bytes));
     if (st.kernels.heavy) {
       const void* hf = (const void*)st.kernels.heavy;
-      DQ_CUDA(cudaFuncSetAttribute(hf, cudaFuncAttributeMaxDynamicSharedMemorySize, st.prog.smem_bytes));
+      allow_smem(hf, st.prog.smem_bytes);
       DQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&st.hocc, hf, st.prog.block, st.prog.smem_bytes));
     }
     if (st.occ < 1 || (st.kernels.heavy && st.hocc < 1)) return nullptr;

@@ -88,3 +88,24 @@ def test_many_domains(engine, dims):
     for _ in range(2):
         assert canonical_rows(p.execute().rows()) == want
     p.free()
+
+
+def test_plans_that_share_a_kernel_over_other_domains(engine):
+    """Their staged bitmaps differ in size, and with them the shared memory of
+    the one kernel: the larger plan runs after the smaller one was prepared."""
+    from dogqc_b200.database import Database, Table
+    from dogqc_b200.lowering import Lowering
+    from helpers import many_domains
+    plans = []
+    for keys in (1 << 18, 1 << 16):
+        db, plan = many_domains(1, keys)
+        lowering = Lowering(plan)
+        for pipe in lowering.pipes:
+            if pipe.table:
+                pipe.table += str(keys)
+        engine.register_database(Database([Table(t.name + str(keys), t.columns, t.types) for t in db.tables.values()]))
+        plans.append((engine.prepare(lowering), canonical_rows(run_plan(db, plan)[1])))
+    assert plans[0][0].source(1) == plans[1][0].source(1)
+    for p, want in plans:
+        assert canonical_rows(p.execute().rows()) == want
+        p.free()

@@ -209,3 +209,35 @@ def test_shared_memory_has_a_budget(engine, dims):
     fact = [plan.source(i) for i in range(dims, len(plan.lowering.pipes))][0]
     assert ("pa0_" in fact) == (dims <= 4)                  # accumulators per thread
     assert fact.count("= __ldcg(g_ + i)") == min(dims, 5)   # staged bitmaps
+
+
+def test_kernels_do_not_depend_on_the_measured_domain(engine):
+    """Plans of one shape over tables of other key ranges share their kernels:
+    a staged bitmap, bits a build side sets for itself, bits of a multimap."""
+    import numpy as np
+    import dogqc_b200.scalar as scal
+    from dogqc_b200.database import Database, Table
+    from dogqc_b200.relational import Reduction
+    from dogqc_b200.types import Type
+    sources = []
+    for keys in (3000, 4900):
+        r = np.random.default_rng(keys)
+        k = r.integers(0, keys, 20_000, dtype=np.int32)
+        k[:2] = (0, keys - 1)
+        db = Database([Table("b", {"k": k, "x": k % 100}, {"k": Type.INT, "x": Type.INT}),
+                       Table("p", {"q": r.integers(0, keys, 20_000, dtype=np.int32)}, {"q": Type.INT})])
+        engine.register_database(db, force=True)
+        for multi in (False, True):
+            alg = RelationalAlgebra(db)
+            if multi:
+                sel = alg.selection(scal.SmallerExpr(scal.AttrExpr("x"), scal.ConstExpr("5", Type.INT)), alg.scan("b"))
+                j = alg.join(("k", "q"), sel, alg.scan("p"))
+                cfg = {sel.opId: {"selectivity": 0.05}}
+            else:
+                j, cfg = alg.semijoin(("k", "q"), None, alg.scan("b"), alg.scan("p")), {}
+            agg = alg.aggregation([], [(Reduction.COUNT, "", "n")], j)
+            plan = engine.prepare(alg.resolveAlgebraPlan(agg, cfg))
+            sources.append([plan.source(i) for i in range(len(plan.lowering.pipes))])
+    semi, multi = "\n".join(sources[0]), "\n".join(sources[1])
+    assert "if (b_) atomicOr" in semi and "= __ldcg(g_ + i)" in semi and ".bits" in multi
+    assert sources[0] == sources[2] and sources[1] == sources[3]
