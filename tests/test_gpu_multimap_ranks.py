@@ -92,6 +92,25 @@ def test_staged_build_side_outgrows_its_estimate(engine, selectivity):
     _check(engine, db, alg.resolveAlgebraPlan(plan, cfg))
 
 
+def _expanding(key, first=0):
+    """400 rows of x meet 500 of y (keys from ``first``; x's are 0 to 9), and
+    the pairs are the build side of a join with p, grouped by ``key`` of x."""
+    from dogqc_b200.database import Database, StringColumn, Table
+    from dogqc_b200.relational import Reduction, RelationalAlgebra
+    from dogqc_b200.types import Type as T
+    r = np.random.default_rng(3)
+    text = [b"name %d" % (i % 11) + b"x" * (i % 40) for i in range(400)]
+    db = Database([Table("x", {"a": r.integers(0, 10, 400, dtype=np.int32), "s": StringColumn.from_list(text),
+                               "t": r.integers(0, 7, 400, dtype=np.int32)}, {"a": T.INT, "s": T.STRING, "t": T.INT}),
+                   Table("y", {"b": r.integers(first, first + 10, 500, dtype=np.int32),
+                               "c": r.integers(0, 20, 500, dtype=np.int32)}, {"b": T.INT, "c": T.INT}),
+                   Table("p", {"d": r.integers(0, 26, 60, dtype=np.int32)}, {"d": T.INT})])
+    alg = RelationalAlgebra(db)
+    pairs = alg.join(("a", "b"), alg.scan("x"), alg.scan("y"))
+    agg = alg.aggregation([key], [(Reduction.COUNT, "", "n")], alg.join(("c", "d"), pairs, alg.scan("p")))
+    return db, alg.resolveAlgebraPlan(agg, {agg.opId: {"numgroups": 400}})
+
+
 @pytest.mark.parametrize("prebuilt", [False, True])
 def test_expanding_build_side_outgrows_its_source(engine, prebuilt):
     """A build side that is itself a multimatch join (and, on generated kernels,
@@ -99,24 +118,10 @@ def test_expanding_build_side_outgrows_its_source(engine, prebuilt):
     the table its pipelines scan: the run ends before a row is placed, the
     payload grows and the run repeats; alone, in a batch and served."""
     import dogqc_b200._lib as L
-    from dogqc_b200.database import Database, StringColumn, Table
     from dogqc_b200.engine import Engine
     from dogqc_b200.lowering import Lowering
-    from dogqc_b200.relational import Reduction, RelationalAlgebra
     from dogqc_b200.serve import Server
-    from dogqc_b200.types import Type as T
-    r = np.random.default_rng(3)
-    text = [b"name %d" % (i % 11) + b"x" * (i % 40) for i in range(400)]
-    db = Database([Table("x", {"a": r.integers(0, 10, 400, dtype=np.int32), "s": StringColumn.from_list(text),
-                               "t": r.integers(0, 7, 400, dtype=np.int32)}, {"a": T.INT, "s": T.STRING, "t": T.INT}),
-                   Table("y", {"b": r.integers(0, 10, 500, dtype=np.int32), "c": r.integers(0, 20, 500, dtype=np.int32)},
-                         {"b": T.INT, "c": T.INT}),
-                   Table("p", {"d": r.integers(0, 26, 60, dtype=np.int32)}, {"d": T.INT})])
-    alg = RelationalAlgebra(db)
-    pairs = alg.join(("a", "b"), alg.scan("x"), alg.scan("y"))
-    key = "t" if prebuilt else "s"
-    agg = alg.aggregation([key], [(Reduction.COUNT, "", "n")], alg.join(("c", "d"), pairs, alg.scan("p")))
-    plan = alg.resolveAlgebraPlan(agg, {agg.opId: {"numgroups": 400}})
+    db, plan = _expanding("t" if prebuilt else "s")
     if prebuilt:
         e = Engine(0, flags=L.CFG_NO_JIT)
         try:
@@ -136,3 +141,16 @@ def test_expanding_build_side_outgrows_its_source(engine, prebuilt):
         assert [canonical_rows(srv.wait(t)[0].rows()) for t in tickets] == [want] * 4
     finally:
         srv.stop()
+
+
+def test_build_side_outgrows_its_source_in_a_replayed_run(engine):
+    """New data makes a replayed run end for want of room; it repeats with room."""
+    (few, plan), (many, _) = _expanding("s", first=9), _expanding("s")
+    engine.register_database(few, force=True)
+    p = engine.prepare(plan)
+    for db in (few, many, few):
+        engine.update_table(db["y"])
+        want = canonical_rows(run_plan(db, plan)[1])
+        for _ in range(4):
+            assert canonical_rows(p.execute().rows()) == want
+    p.free()
