@@ -1267,6 +1267,12 @@ struct Gen {
       L("if (lane == dl_) db_ = atomicAdd(P.heavy.count, (uint32_t)__popc(dm_));");
       L("db_ = __shfl_sync(kFull, db_, dl_);");
       L("const uint32_t hs_ = db_ + (uint32_t)__popc(dm_ & ((1u << lane) - 1u));");
+      if (!batched) {
+        L("if (P.heavy.cap == 0u && " + ec + " > kWideRange) {");
+        L("  set_status(P, kErrWideRange);");
+        L("  " + ec + " = 0u;");
+        L("}");
+      }
       L("if (dw_ && hs_ < P.heavy.cap) {");
       ++ind;
       L("uint64_t* it_ = P.heavy.items + (size_t)hs_ * P.heavy.words;");

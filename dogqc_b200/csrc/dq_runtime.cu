@@ -1594,6 +1594,8 @@ int run_once(dq_plan* plan, cudaStream_t st) {
       if (pp->clears_source) plan->res[pp->desc.source_res]->agg_clean = true;
     plan->steady = true;
   } else {
+    // a kernel that ended the run may have filled tables its scans then left alone
+    for (auto& rp : plan->res) rp->agg_clean = false;
     plan->steady = false;
     plan->drop_graph();
   }
@@ -2108,7 +2110,8 @@ void adapt_threshold(dq_plan* plan) {
     PipeRec& p = *pp;
     if (p.expand_op < 0 || !p.stats_read || !p.dev.heavy.grouped) continue;
     // Two runs without a deferred range: the runs that follow have no room for
-    // items (cap 0: a longer range is counted and expanded in place) and none of
+    // items (cap 0: a longer range is counted and expanded in place, one of more
+    // than kWideRange rows ends the run, which is repeated with room) and none of
     // the deferral's four launches, until one counts a range again (Q13 shape:
     // 204 us a pass with them, 188 without; Q22 shape: 89 and 78).
     const bool was_off = p.heavy_off();
@@ -2130,6 +2133,17 @@ void adapt_threshold(dq_plan* plan) {
       ++plan->epoch;
     }
   }
+}
+
+// After a run that met a range too long to expand in place: all of the plan's
+// expansions defer again.
+void defer_again(dq_plan* plan) {
+  for (auto& pp : plan->pipes) {
+    if (pp->expand_op < 0 || !pp->heavy_off()) continue;
+    pp->heavy_empty = 0;
+    pp->dev.heavy.cap = pp->heavy_full;
+  }
+  ++plan->epoch;
 }
 
 void throw_status(int status) {
@@ -2854,7 +2868,8 @@ int dq_plan_execute(dq_plan* plan, void* stream, dq_result** out) {
                       : status & (kErrOverflow | kErrMultiFull) ? DQ_ERR_OVERFLOW : DQ_ERR_BAD_IR,
                       "device status " + std::to_string(status));
       // grow what overflowed and run again (the results of a failed run are discarded)
-      grow_plan(plan, status);
+      if (status & kErrWideRange) defer_again(plan);
+      if (status & ~kErrWideRange) grow_plan(plan, status);
     }
     *out = take_result(plan, st);
     return (int)DQ_OK;

@@ -24,16 +24,20 @@ def _db(skew, seed):
                            {"q": Type.INT, "y": Type.INT})])
 
 
-def test_long_ranges_come_and_go():
+def _plan(db):
     import dogqc_b200.scalar as scal
-    from dogqc_b200.engine import Engine
     from dogqc_b200.relational import Reduction, RelationalAlgebra
-    dbs = [_db(0, 1), _db(5000, 2)]
-    alg = RelationalAlgebra(dbs[0])
+    alg = RelationalAlgebra(db)
     j = alg.join(("k", "q"), alg.scan("b"), alg.scan("p"))
     sel = alg.selection(scal.SmallerExpr(scal.AttrExpr("x"), scal.AttrExpr("y")), j)
     agg = alg.aggregation([], [(Reduction.COUNT, "", "n"), (Reduction.SUM, "m", "s")], sel)
-    plan = alg.resolveAlgebraPlan(agg, {})
+    return alg.resolveAlgebraPlan(agg, {})
+
+
+def test_long_ranges_come_and_go():
+    from dogqc_b200.engine import Engine
+    dbs = [_db(0, 1), _db(5000, 2)]
+    plan = _plan(dbs[0])
     want = [canonical_rows(run_plan(db, plan)[1]) for db in dbs]
     e = Engine(0)
     try:
@@ -49,6 +53,34 @@ def test_long_ranges_come_and_go():
         assert launches[4] == launches[0] - 4    # long after two runs that deferred nothing
         assert launches[9] == launches[0]
         assert launches[14] == launches[4] and launches[19] == launches[0]
+        p.free()
+    finally:
+        e.close()
+
+
+def test_a_very_long_range_is_not_expanded_in_place():
+    """A range of more than 2^11 rows in a run without the deferral: that run
+    ends and is repeated with it."""
+    from dogqc_b200.engine import Engine
+    dbs = [_db(0, 1), _db(2000, 2), _db(2100, 3)]
+    plan = _plan(dbs[0])
+    e = Engine(0)
+    try:
+        e.register_database(dbs[0])
+        p = e.prepare(plan)
+        full = None
+        for turn, db in enumerate((dbs[0], dbs[1], dbs[0], dbs[2], dbs[0])):
+            for t in db.tables.values():
+                e.update_table(t)
+            want = canonical_rows(run_plan(db, plan)[1])
+            launches = []
+            for _ in range(5):
+                assert canonical_rows(p.execute().rows()) == want
+                launches.append(p.timing()["kernel_launches"])
+            full = full or launches[0]
+            # the first run over changed data: in place up to 2^11 rows, else with the deferral
+            assert launches[0] == (full - 4 if turn == 1 else full)
+            assert launches[4] == (full - 4 if db is dbs[0] else full)
         p.free()
     finally:
         e.close()
