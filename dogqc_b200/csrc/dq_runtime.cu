@@ -1720,7 +1720,7 @@ dq_result* read_result(dq_plan* plan, cudaStream_t st) {
 
 // Device bytes a plan holds (its tables, intermediates and scratch).
 uint64_t plan_bytes(const dq_plan* plan) {
-  uint64_t b = plan->status.bytes;
+  uint64_t b = plan->status.bytes + plan->str_lens.bytes + plan->str_offs.bytes + plan->str_heap.bytes;
   for (auto& rp : plan->res) {
     const ResRec& r = *rp;
     b += r.slots.bytes + r.counts.bytes + r.ranges.bytes + r.scan_scratch.bytes + r.rank.bytes +
@@ -3913,6 +3913,9 @@ PoolEntry* srv_acquire(dq_server* s, SrvReq* r) {
 
 void srv_release(dq_server* s, SrvReq* r, PoolEntry* pe) {
   pe->busy = false;
+  const uint64_t before = pe->bytes;
+  pe->bytes = plan_bytes(pe->plan.get());  // with the scratch its string results took
+  s->mem = s->mem - before + pe->bytes;
   auto& v = s->pool[r->desc->key];
   int idle = 0;
   for (auto& e : v) idle += !e->busy;

@@ -206,3 +206,31 @@ def test_string_requests_alone_and_batched(engine):
                 assert srv.stats()["batches"] > 0
         finally:
             srv.stop()
+
+
+def test_string_result_scratch_counts_as_the_plans_memory(engine):
+    """A pooled plan keeps the buffers its string columns are gathered in: they
+    are part of the memory the server accounts for."""
+    import numpy as np
+    from dogqc_b200 import serve
+    from dogqc_b200.database import Database, StringColumn, Table
+    from dogqc_b200.lowering import Lowering
+    from dogqc_b200.relational import RelationalAlgebra
+    from dogqc_b200.types import Type
+    text = [b"%06d" % i * 20 for i in range(30_000)]
+    db = Database([Table("texts", {"i": np.arange(30_000, dtype=np.int32), "s": StringColumn.from_list(text)},
+                         {"i": Type.INT, "s": Type.STRING})])
+    engine.register_database(db)
+    alg = RelationalAlgebra(db)
+    plan = alg.resolveAlgebraPlan(alg.projection(["i", "s"], alg.scan("texts")), {})
+    srv = serve.Server(engine, slots=1, pool_per_query=1)
+    try:
+        used = []
+        for _ in range(3):
+            res, info = srv.wait(srv.submit(Lowering(plan)))
+            assert sorted(res.rows()) == list(enumerate(text))
+            used.append(info["bytes"])
+        assert used[1] == used[2] >= used[0] + sum(map(len, text)) + 2 * 8 * len(text)
+        assert srv.stats()["memory_in_use"] == used[2]
+    finally:
+        srv.stop()
