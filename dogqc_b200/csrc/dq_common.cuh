@@ -292,21 +292,23 @@ __device__ __forceinline__ bool like_find(const uint8_t* s, int n, int& pos, con
   return false;
 }
 
-// Which of the warp's strings can hold a literal L of m >= 3 bytes: those with
-// its first min(m, 4) bytes in them, m bytes from their end or earlier.  The
-// lanes' strings are consecutive in one heap (rows row0 + lane; `in`: a lane has
-// one, lane 0 does), so the warp reads their bytes as one range, 16 a lane, and
-// compares the literal's first bytes at every position; the few that agree are
-// given to the lane whose string they lie in.  Bytes come coalesced and every
-// lane works, whatever the strings' lengths (1.5 M comments of 57 bytes searched
-// for two words: 157 -> 67 us).  Loads stay within 16 bytes of the
-// range (heaps start 256-byte aligned and are padded at the end).
+// Which of the warp's strings hold a literal L of m >= 3 bytes.  The lanes'
+// strings are consecutive in one heap (rows row0 + lane; `in`: a lane has one,
+// the lowest ones do), so the warp reads their bytes as one range, 16 a lane, and
+// compares the literal's first bytes at every position.  Positions that agree
+// are taken one a lane and round: the lane finds the string they lie in and
+// compares the rest.  Bytes come coalesced and every lane works, whatever the
+// strings' lengths.  Device us of a scan, a lane a string / this: 1.5 M strings of
+// 57 bytes 64 / 59 without a hit, 52 / 102 with two hits a string, where a lane's
+// own search ends early (192 when the warp took the positions one by one);
+// 200,000 of 500 bytes 186 / 79 and 88 / 87.  Loads stay within 16 bytes of the range (heaps start 256-byte
+// aligned and are padded at the end).
 __device__ __noinline__ bool like_candidates(bool in, const uint8_t* s, int n, const uint8_t* L, int m) {
   const int lane = (int)(threadIdx.x & 31);
-  const unsigned have = __ballot_sync(kFull, in);
+  const int count = __popc(__ballot_sync(kFull, in));
   const unsigned long long at = (unsigned long long)s;
   const unsigned long long first = __shfl_sync(kFull, at, 0);
-  const unsigned long long end = __shfl_sync(kFull, at + (unsigned long long)n, 31 - __clz(have));
+  const unsigned long long end = __shfl_sync(kFull, at + (unsigned long long)n, count - 1);
   uint32_t key = (uint32_t)L[0] | (uint32_t)L[1] << 8 | (uint32_t)L[2] << 16;
   const uint32_t mask = m >= 4 ? 0xffffffffu : 0xffffffu;
   if (m >= 4) key |= (uint32_t)L[3] << 24;
@@ -322,11 +324,25 @@ __device__ __noinline__ bool like_candidates(bool in, const uint8_t* s, int n, c
 #pragma unroll
     for (int b = 0; b < 16; ++b)
       if ((((b & 3) ? __funnelshift_r(x[b >> 2], x[(b >> 2) + 1], 8 * (b & 3)) : x[b >> 2]) & mask) == key) cand |= 1u << b;
-    for (unsigned todo = __ballot_sync(kFull, cand != 0); todo; todo = __ballot_sync(kFull, cand != 0)) {
-      const int src = __ffs(todo) - 1;
-      const unsigned long long c = __shfl_sync(kFull, a + (unsigned long long)(__ffs(cand) - 1), src);
-      if (lane == src) cand &= cand - 1;
-      hit = hit || (in && c >= at && c + m <= at + n);
+    if (__any_sync(kFull, cand != 0)) {
+      // where this lane's string starts and ends, from pos on
+      const int rs = at <= pos ? 0 : (int)(at - pos < 1024 ? at - pos : 1024);
+      const int re = at + n <= pos ? 0 : (int)(at + n - pos < (1u << 30) ? at + n - pos : 1u << 30);
+      do {
+        const int c = 16 * lane + (cand ? __ffs(cand) - 1 : 0);
+        int o = 0;  // the last string that starts at c or before (empty ones before it may start there too)
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+          const int t = __shfl_sync(kFull, rs, (o + d) & 31);
+          if (o + d < count && t <= c) o += d;
+        }
+        bool ok = __shfl_sync(kFull, rs, o) <= c;
+        ok = c + m <= __shfl_sync(kFull, re, o) && ok && cand != 0;
+        for (int j = 4; ok && j < m; ++j) ok = reinterpret_cast<const uint8_t*>(pos)[c + j] == L[j];
+        const unsigned holds = __reduce_or_sync(kFull, ok ? 1u << o : 0u);  // (every lane takes part)
+        hit = hit || ((holds >> lane) & 1u);
+        cand &= cand - 1;
+      } while (__any_sync(kFull, cand != 0));
     }
     if (__all_sync(kFull, hit || !in || n < m)) break;
   }

@@ -635,7 +635,7 @@ struct Gen {
         case DQ_OP_LIKE: {
           // a pattern '%L1%...%Ln%' (no '_', no empty literal) finds its
           // literals one after another, eight bytes a step, in the strings
-          // that can hold one of them; others run the reference matcher's
+          // that hold one of them; others run the reference matcher's
           // algorithm (like_match)
           const std::vector<std::pair<int, int>> lits = like_literals(op.res);
           const bool simple = !lits.empty();
@@ -648,6 +648,10 @@ struct Gen {
             L("if (__any_sync(kFull, " + act + "))");
             L("  lc" + id + "_ = like_candidates(" + act + ", lk" + id + "_, ln" + id + "_, P.patterns + " + num(lits[(size_t)scan].first) +
               ", " + num(lits[(size_t)scan].second) + ");");
+            if (lits.size() == 1) {  // holding it is all the pattern asks
+              L(V(op.dst) + " = lc" + id + "_ ? 1ull : 0ull;");
+              break;
+            }
             L(V(op.dst) + " = 0;");
             L("if (lc" + id + "_) {");
             ++ind;
