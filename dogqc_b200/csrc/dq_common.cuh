@@ -301,8 +301,8 @@ __device__ __forceinline__ bool like_find(const uint8_t* s, int n, int& pos, con
 // strings' lengths.  Device us of a scan, a lane a string / this: 1.5 M strings of
 // 57 bytes 64 / 59 without a hit, 52 / 102 with two hits a string, where a lane's
 // own search ends early (192 when the warp took the positions one by one);
-// 200,000 of 500 bytes 186 / 79 and 88 / 87.  Loads stay within 16 bytes of the range (heaps start 256-byte
-// aligned and are padded at the end).
+// 200,000 of 500 bytes 186 / 79 and 88 / 87.  Loads stay within 16 bytes of the
+// range (heaps start 256-byte aligned and are padded at the end).
 __device__ __noinline__ bool like_candidates(bool in, const uint8_t* s, int n, const uint8_t* L, int m) {
   const int lane = (int)(threadIdx.x & 31);
   const int count = __popc(__ballot_sync(kFull, in));

@@ -558,7 +558,7 @@ struct Gen {
   // The literal of LIKE op k that the whole warp looks for first (an index into
   // its literals), or -1: the op reads a column in place before any operator
   // has dropped rows, so the warp's lanes hold consecutive strings (one row a
-  // lane and step: generate() then takes U = 1), and the literal has at least
+  // lane and step: choose() then takes U = 1), and the literal has at least
   // three bytes.
   int scan_literal(int k) const {
     const dq_op& op = P.ops[k];
@@ -2725,9 +2725,10 @@ static Gen choose(const DevPipe& P, int expand_op, int refill_op, const Tuning& 
   if (t.refill < 0) refill_op = -1;
   if (t.refill_threshold >= 1 && t.refill_threshold <= 32) g.refill_threshold = t.refill_threshold;
   // strings searched by the whole warp: consecutive rows on consecutive lanes
+  // (asked for more rows a thread, a lane searches its own)
   bool scans = false;
   for (int k = 0; k < P.nops; ++k) scans |= g.scan_literal(k) >= 0;
-  if (scans) g.U = 1;
+  if (rows <= 0 && scans) g.U = 1;
   // string keys: a row waits for its strings' offsets, then for their bytes, so
   // more warps hide more of that than more rows a thread, whose registers the
   // strings' words multiply (6 M rows grouped by two strings: one row a thread

@@ -241,3 +241,15 @@ def test_kernels_do_not_depend_on_the_measured_domain(engine):
     semi, multi = "\n".join(sources[0]), "\n".join(sources[1])
     assert "if (b_) atomicOr" in semi and "= __ldcg(g_ + i)" in semi and ".bits" in multi
     assert sources[0] == sources[2] and sources[1] == sources[3]
+
+
+@pytest.mark.parametrize("rows", [None, 1, 2, 4])
+def test_rows_per_thread_reach_a_like_scan(engine, rows):
+    """The warp-wide search takes one row a thread; a tuning that asks for more
+    gets them, with a search a lane."""
+    plan = engine.prepare(resolved(engine, "c17"), tuning={"rows_per_thread": rows} if rows else None)
+    src = [plan.source(i) for i in range(len(plan.lowering.pipes)) if "str_at" in plan.source(i)]
+    src = [s[:s.index("compiler report")] for s in src]
+    assert len(src) == 1
+    assert ("like_candidates" in src[0]) == (rows in (None, 1))
+    assert "u < %d; ++u" % (rows or 1) in src[0]
