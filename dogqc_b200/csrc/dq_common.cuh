@@ -507,6 +507,8 @@ __device__ __forceinline__ void str_words_short(const uint8_t* p, int n, uint64_
 
 // A 32-bit hash of a short string from its words (a multilinear hash: one
 // multiply-add a 32-bit word), for CTA-local tables that compare the strings.
+// The multipliers only have to be odd and unlike one another; they are constants
+// of well-known public hashes (2^32 over the golden ratio, MurmurHash3, xxHash32).
 __device__ __forceinline__ uint32_t str_hash32_words(const uint64_t* w, int n) {
   uint32_t h = (uint32_t)n * 0x9e3779b1u;
   h += (uint32_t)w[0] * 0x85ebca77u + (uint32_t)(w[0] >> 32) * 0xc2b2ae3du;
