@@ -2732,13 +2732,16 @@ static Gen choose(const DevPipe& P, int expand_op, int refill_op, const Tuning& 
   // string keys: a row waits for its strings' offsets, then for their bytes, so
   // more warps hide more of that than more rows a thread, whose registers the
   // strings' words multiply (6 M rows grouped by two strings: one row a thread
-  // 184 us at 80 registers, two 225 us at 116, four 323 us at 120)
+  // 184 us at 80 registers, two 225 us at 116, four 323 us at 120; joins on a
+  // string key, the whole plan with one, two, four rows: unique 29 / 32 / 42 us,
+  // semi 31 / 37 / 48, with a condition 197 / 203 / 248, multimatch 307 / 308 / 311)
   if (rows <= 0 && g.string_keys()) g.U = 1;
   g.choose_agg();
   // a CTA merges its group table into the global one at its end, an atomic per
   // group and accumulator on the same few addresses as every other CTA: twice
   // the threads a CTA, half the merges (6 M probes into 25 groups of two, 256
-  // threads 49.8 us, 512 43.3)
+  // threads 49.8 us, 512 43.3; scans of 6 M rows into 17 to 128 groups of one to
+  // five aggregates: 512 threads take 0.91 to 1.02 of 256's time)
   if (g.agg == AGG_STRIPED && P.res[g.agg_res].packed && t.block == 0 && !t.batched && frugal < 2) g.block = 512;
   g.choose_refill(refill_op);
   g.choose_hot();
