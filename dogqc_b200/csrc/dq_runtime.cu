@@ -528,11 +528,11 @@ void host_range(ColRec& rec, const dq_column& c, int64_t nrows) {
   }
 }
 
-void upload_column(dq_ctx* ctx, ColRec& rec, const dq_column& c, int64_t nrows, bool device_src,
+void upload_column(dq_ctx* ctx, ColRec& rec, const dq_column& c, int64_t nrows, int32_t flags,
                    cudaStream_t stream) {
-  cudaMemcpyKind kind = device_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  if (ctx->offline) {  // sizes and value ranges only
-    if (!device_src) host_range(rec, c, nrows);
+  cudaMemcpyKind kind = flags & DQ_TABLE_DEVICE_DATA ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+  if (ctx->offline) {  // sizes and, asked for, value ranges only
+    if ((flags & DQ_TABLE_KEY_RANGES) && !(flags & DQ_TABLE_DEVICE_DATA)) host_range(rec, c, nrows);
     if (!rec.data) rec.data = std::make_shared<DevBuf>();
     if (c.ctype == DQ_STR && c.width <= 0 && !rec.offsets) rec.offsets = std::make_shared<DevBuf>();
     return;
@@ -2471,7 +2471,7 @@ int dq_table_register(dq_ctx* ctx, const char* name, int32_t ncols, const dq_col
       rec.name = c.name;
       rec.ctype = c.ctype;
       rec.width = c.ctype == DQ_STR ? c.width : ctype_width(c.ctype);
-      upload_column(ctx, rec, c, nrows, flags & DQ_TABLE_DEVICE_DATA, ctx->stream);
+      upload_column(ctx, rec, c, nrows, flags, ctx->stream);
       t.cols.push_back(std::move(rec));
     }
     if (!ctx->offline) DQ_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -271,7 +271,8 @@ class Engine(object):
 
     def register_table(self, table):
         arr, n, keep = self._columns(table)
-        L.check(L.lib().dq_table_register(self.ctx, table.name.encode(), n, arr, table.size, 0), self.ctx)
+        L.check(L.lib().dq_table_register(self.ctx, table.name.encode(), n, arr, table.size, L.TABLE_KEY_RANGES),
+                self.ctx)
         self.registered[table.name] = table
 
     def register_database(self, db, force=False):

@@ -100,6 +100,10 @@ typedef struct {
 } dq_column;
 
 #define DQ_TABLE_DEVICE_DATA 1  /* pointers are device memory (else host)      */
+#define DQ_TABLE_KEY_RANGES  2  /* offline contexts: read the integer columns' */
+                                /* smallest and largest values from the host   */
+                                /* data (else no column is read: plans are     */
+                                /* compiled without key-domain tables)         */
 
 /* Copies the columns into library-owned, padded device memory (replacing a
  * table of the same name).                                                   */

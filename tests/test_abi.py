@@ -60,3 +60,19 @@ def test_noalloc_rejects_bad_arguments_before_any_device_work(field, value, need
     setattr(a, field, L.NOALLOC_MAX_GROUPS + 1 if value is None else value)
     assert lib.dq_join_agg_noalloc(C.byref(a), None) == L.ERR_INVALID
     assert needle in lib.dq_last_error(None)
+
+
+def test_offline_tables_are_metadata():
+    """An offline context reads no column unless it is asked for key ranges."""
+    import ctypes as C
+    from dogqc_b200 import _lib as L
+    from dogqc_b200.engine import Engine
+    e = Engine(0, flags=L.CFG_OFFLINE)
+    try:
+        col = (L.dq_column * 1)()
+        col[0].name, col[0].ctype, col[0].data = b"k", L.I32, 16   # no such memory
+        assert L.lib().dq_table_register(e.ctx, b"t", 1, col, 1000, 0) == L.OK
+        n = C.c_int64()
+        assert L.lib().dq_table_rows(e.ctx, b"t", C.byref(n)) == L.OK and n.value == 1000
+    finally:
+        e.close()
