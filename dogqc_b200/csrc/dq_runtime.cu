@@ -838,11 +838,14 @@ void check_smem(const jit::Program& prog) {
 // kernel's limit only ever grows.
 void allow_smem(const void* fn, int bytes) {
   static std::mutex mu;
+  static std::map<std::pair<int, const void*>, int> limits;  // (kernels stay loaded)
+  int device = 0;
+  DQ_CUDA(cudaGetDevice(&device));
   std::lock_guard<std::mutex> lk(mu);
-  cudaFuncAttributes a;
-  DQ_CUDA(cudaFuncGetAttributes(&a, fn));
-  if (a.maxDynamicSharedSizeBytes < bytes)
-    DQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  const auto it = limits.emplace(std::make_pair(device, fn), -1).first;
+  if (it->second >= bytes) return;
+  DQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  it->second = bytes;
 }
 
 void setup_pipeline(dq_plan* plan, PipeRec& p) {
