@@ -1095,7 +1095,7 @@ struct Gen {
     if (R.row_bytes <= 0 || R.npay <= 0) return;
     const std::string T = item_type(R.row_bytes), v = fresh("gi");
     L(T + " " + v + " = " + (R.row_bytes == 16 ? "make_uint4(0u, 0u, 0u, 0u)" : R.row_bytes == 8 ? "make_uint2(0u, 0u)" : "0u") + ";");
-    L("if (" + act + ") " + v + " = reinterpret_cast<const " + T + "*>(" + res(r) + ".pay[" + num(item_base(r)) + "])[" + m + "];");
+    L("if (" + act + ") " + v + " = __ldg(reinterpret_cast<const " + T + "*>(" + res(r) + ".pay[" + num(item_base(r)) + "]) + " + m + ");");
     item[r] = v;
   }
 
