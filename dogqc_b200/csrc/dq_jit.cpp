@@ -1089,13 +1089,16 @@ struct Gen {
   static const char* item_type(int bytes) { return bytes == 16 ? "uint4" : bytes == 8 ? "uint2" : "uint32_t"; }
 
   // Loads the payload item of match `m` of multimap r (one load) when its rows
-  // are items; gather() then takes its fields.
-  void gather_item(int r, const std::string& act, const std::string& m) {
+  // are items; gather() then takes its fields.  A lane's walk of a range reads it
+  // through the read-only path (50,000 rows walked: 4.2 ms, 6.2 with plain loads),
+  // an expansion's pairs do not (256 batched expansions: 1.10 ms, 1.12 with).
+  void gather_item(int r, const std::string& act, const std::string& m, bool walk = false) {
     const DevRes& R = P.res[r];
     if (R.row_bytes <= 0 || R.npay <= 0) return;
     const std::string T = item_type(R.row_bytes), v = fresh("gi");
     L(T + " " + v + " = " + (R.row_bytes == 16 ? "make_uint4(0u, 0u, 0u, 0u)" : R.row_bytes == 8 ? "make_uint2(0u, 0u)" : "0u") + ";");
-    L("if (" + act + ") " + v + " = __ldg(reinterpret_cast<const " + T + "*>(" + res(r) + ".pay[" + num(item_base(r)) + "]) + " + m + ");");
+    L("if (" + act + ") " + v + " = " + (walk ? "__ldg(" : "*(") + "reinterpret_cast<const " + T + "*>(" + res(r) + ".pay[" +
+      num(item_base(r)) + "]) + " + m + ");");
     item[r] = v;
   }
 
@@ -1213,7 +1216,7 @@ struct Gen {
     const std::vector<std::string> saved = var;
     const std::map<int, std::string> saved_item = item;
     item.clear();
-    gather_item(r, "true", m);
+    gather_item(r, "true", m, true);
     for (int s2 = 0; s2 < P.nslots; ++s2)
       if (slot(s2).kind == DQ_SLOT_GATHER && slot(s2).level == lv && slot(s2).res == r) gather(s2, "true", m);
     std::string eq = "true";
