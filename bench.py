@@ -265,6 +265,7 @@ def run_ours(args, world, rank, local):
     def flush_l2():
         flush.fill_(1)
         evict.sum()
+        torch.cuda.synchronize()  # the run must not share the device with the flush
 
     # the plan's launch shapes and table sizing, picked by measurement on this
     # GPU (each candidate run after an L2 flush) before anything is timed
@@ -288,7 +289,6 @@ def run_ours(args, world, rank, local):
         per-pipeline times (zero where the run replayed a graph), launches."""
         def step():
             flush_l2()
-            torch.cuda.synchronize()
             res_ = plan_.execute()
             return res_, plan_.timing()
         for _ in range(args.warmup):

@@ -133,7 +133,8 @@ def batch_measure(engine, lowerings, reps=3, warmup=1):
 def plan_measure(engine, lowering, reps=3, warmup=1, between=None):
     """Median device time of a plan prepared with the candidate tuning;
     ``between()`` runs before every execution (an L2 flush, so that inputs
-    that would fit L2 are read from HBM as in a timed run)."""
+    that would fit L2 are read from HBM as in a timed run) and returns when the
+    device has finished it."""
     def measure(tuning):
         try:
             p = engine.prepare(lowering, tuning=tuning)
